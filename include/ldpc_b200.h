@@ -421,6 +421,14 @@ int ldpc_probe_fp32_peak(int device, double *fma_per_s, double *mufu_per_s);
  * static string naming operation i.  No counterpart in the reference. */
 int ldpc_probe_op_rates(int device, double *ops_per_clk_sm, int n_ops, const char **names);
 
+/* Compares the decoders' branch-free tanh(a/2) and 2 atanh(m) (sp_math.cuh)
+ * with the functions shared with the CPU oracle (ldpc_math.h) on `device`: in
+ * float on every a in [0, inf] and every m in [0, 1], in double on `samples`
+ * random and boundary arguments of each per GPU thread (303104 threads).
+ * *mismatches receives the number of results that differ in any bit.  No
+ * counterpart in the reference. */
+int ldpc_probe_sp_math(int device, int samples, unsigned long long *mismatches);
+
 #ifdef __cplusplus
 }
 #endif

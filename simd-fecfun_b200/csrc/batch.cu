@@ -137,6 +137,10 @@ struct PlanDel {
     void operator()(ldpc_batch_plan* p) const { destroy_plan(p); }
 };
 
+// shared memory of a float batch CTA: the float decoders' limit for everything but
+// the code's tables, whose circulants are 8 bytes each
+constexpr int kSpBatchSmem = ldpc::kSpMaxSmem + ldpc::SP_MAX_E * 2;
+
 int float_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads, int cpc, ldpc_batch_plan** out) {
     const int nc = (int)b->codes.size();
     const bool prod = b->variant == LDPC_F32_SP;
@@ -152,15 +156,15 @@ int float_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int thread
         const int n = cd.z * cd.mcol, E = (int)cd.row_cols.size();
         auto bytes = [&](int g) {
             ldpc::SpTables t;
-            ldpc::fill_sp_tables(cd, g, &t);
+            ldpc::fill_sp_tables(cd, g, (int)sizeof(float), &t);
             return (size_t)ldpc::sp_code_bytes() + (((size_t)g * t.stride + 3) & ~(size_t)3) * 4 + (size_t)g * ((n + 3) & ~3) * 4;
         };
         G[c] = std::max(1, std::min(32, threads / cd.z));
-        while (G[c] > 1 && bytes(G[c]) > (size_t)ldpc::kSpMaxSmem) --G[c];
+        while (G[c] > 1 && bytes(G[c]) > (size_t)kSpBatchSmem) --G[c];
         base[c] = bytes(G[c]);
-        if (base[c] > (size_t)ldpc::kSpMaxSmem)
+        if (base[c] > (size_t)kSpBatchSmem)
             return fail(LDPC_ERR_UNSUPPORTED, "batch plan: code %d (N=%d) does not fit shared memory", c, n);
-        if (base[c] + (size_t)(E | 1) * threads * 4 > (size_t)ldpc::kSpMaxSmem) rsmem = false;   // odd per-thread stride
+        if (base[c] + (size_t)(E | 1) * threads * 4 > (size_t)kSpBatchSmem) rsmem = false;   // odd per-thread stride
         dmax = std::max(dmax, cd.max_row_weight <= 8 ? 8 : cd.max_row_weight <= 16 ? 16 : 32);
         maxE = std::max(maxE, E);
     }
@@ -180,8 +184,8 @@ int float_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int thread
         // as for a single code: sum-product keeps shared-memory messages
         // unless global (L2) messages give at least 1.5 times the CTAs per SM
         int per_s = 0, per_g = 0;
-        CUDA_TRY(ldpc::allow_dynamic_smem((const void*)find(true), ldpc::kSpMaxSmem));
-        CUDA_TRY(ldpc::allow_dynamic_smem((const void*)find(false), ldpc::kSpMaxSmem));
+        CUDA_TRY(ldpc::allow_dynamic_smem((const void*)find(true), kSpBatchSmem));
+        CUDA_TRY(ldpc::allow_dynamic_smem((const void*)find(false), kSpBatchSmem));
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_s, (const void*)find(true), threads, smem_of(true)));
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_g, (const void*)find(false), threads, smem_of(false)));
         rsmem = 2 * per_g < 3 * per_s;
@@ -194,7 +198,7 @@ int float_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int thread
     p->kf = (void*)k;
     p->threads = threads;
     p->smem = (int)smem;
-    CUDA_TRY(ldpc::allow_dynamic_smem((const void*)k, ldpc::kSpMaxSmem));
+    CUDA_TRY(ldpc::allow_dynamic_smem((const void*)k, kSpBatchSmem));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, threads, smem));
     if (per_sm < 1) return fail(LDPC_ERR_UNSUPPORTED, "batch plan: %d threads x %zu B do not fit an SM", threads, smem);
@@ -202,7 +206,7 @@ int float_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int thread
     std::vector<ldpc::SpCode> hc(nc);
     for (int c = 0; c < nc; ++c) {
         memset(&hc[c], 0, sizeof(hc[c]));
-        ldpc::fill_sp_tables(b->codes[c], G[c], &hc[c].t);
+        ldpc::fill_sp_tables(b->codes[c], G[c], (int)sizeof(float), &hc[c].t);
         hc[c].max_iter = (int)b->cfgs[c].max_iter;
         hc[c].num_par = b->codes[c].num_par;
         hc[c].beta = b->cfgs[c].beta;

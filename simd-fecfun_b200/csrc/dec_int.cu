@@ -47,10 +47,7 @@ int setup_int(ldpc_ctx* x) {
         t.ebase[l] = (int16_t)e0;
         e0 += c.row_weights[l];
     }
-    for (int e = 0; e < t.E; ++e) {
-        t.colz[e] = c.row_cols[e] * c.z;
-        t.shift[e] = (int16_t)c.row_shifts[e];
-    }
+    for (int e = 0; e < t.E; ++e) t.edge[e] = {4u * (uint32_t)(c.row_cols[e] * c.z), 4u * (uint32_t)(c.row_shifts[e] - c.z)};
     int G = std::max(1, std::min(32, 128 / c.z));
     while (G > 1 && ((G * c.z + 31) / 32) * 32 > kIntMaxThreads) --G;
     t.G = G;

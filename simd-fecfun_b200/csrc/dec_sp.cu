@@ -26,7 +26,7 @@ const SpVariant kSp[] = {
 bool is_f64(int variant) { return variant == LDPC_F64_SP || variant == LDPC_F64_OMS; }
 }  // namespace
 
-void fill_sp_tables(const ldpc_code& c, int G, SpTables* out) {
+void fill_sp_tables(const ldpc_code& c, int G, int es, SpTables* out) {
     SpTables& t = *out;
     memset(&t, 0, sizeof(t));
     t.z = c.z;
@@ -42,10 +42,8 @@ void fill_sp_tables(const ldpc_code& c, int G, SpTables* out) {
         t.ebase[l] = (int16_t)e0;
         e0 += c.row_weights[l];
     }
-    for (int e = 0; e < t.E; ++e) {
-        t.colz[e] = c.row_cols[e] * c.z;
-        t.shift[e] = (int16_t)c.row_shifts[e];
-    }
+    for (int e = 0; e < t.E; ++e)
+        t.edge[e] = {(uint32_t)es * (uint32_t)(c.row_cols[e] * c.z), (uint32_t)es * (uint32_t)(c.row_shifts[e] - c.z)};
     t.G = G;
     t.stride = t.n + ((((32 + G - 1) / G) - t.n) % 32 + 32) % 32;
 }
@@ -70,13 +68,14 @@ int setup_sp(ldpc_ctx* x) {
     // exceeds the shared memory, then no staging buffer
     const int nstage = (c.z * c.mcol + V - 1) & ~(V - 1);
     auto base_bytes = [&](int g, bool stage) {
-        fill_sp_tables(c, g, &t);
+        fill_sp_tables(c, g, (int)es, &t);
         return ((((size_t)g * t.stride + V - 1) & ~(size_t)(V - 1)) + (stage ? (size_t)g * nstage : 0)) * es;
     };
     while (G > 1 && base_bytes(G, true) > (size_t)kSpMaxSmem) --G;
     const bool nostage = base_bytes(G, true) > (size_t)kSpMaxSmem;
     const size_t base_smem = base_bytes(G, !nostage);   // leaves t filled for G
     t.nostage = nostage ? 1 : 0;
+    const int edge_smem = sp_edge_bytes(t.E);
     x->sp_threads = ((G * c.z + 31) / 32) * 32;
     // messages: shared memory holds E | 1 per thread (odd stride), the global
     // scratch E per thread
@@ -96,8 +95,9 @@ int setup_sp(ldpc_ctx* x) {
     };
     auto ctas_per_sm = [&](const SpVariant* k, size_t bytes, int* out) -> cudaError_t {
         const void* fn = dbl ? (const void*)k->k64 : (const void*)k->k;
-        cudaError_t e = allow_dynamic_smem(fn, kSpMaxSmem);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, fn, x->sp_threads, bytes);
+        cudaError_t e = allow_dynamic_smem(fn, kSpMaxSmem + kSpEdgeSmem);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, fn, x->sp_threads, bytes + edge_smem);
         return e;
     };
     // tuning: LDPC_SP_RGLOBAL forces global messages, LDPC_SP_RSMEM shared
@@ -114,10 +114,11 @@ int setup_sp(ldpc_ctx* x) {
     x->sp64_kernel = dbl ? v->k64 : nullptr;
     const void* kfn = dbl ? (const void*)v->k64 : (const void*)v->k;
     x->sp_smem = (int)(base_smem + (rsmem ? r_smem : 0));
-    // up to 220 KB dynamic (B200: 227 KB per CTA, less the kernel's static shared memory)
+    // up to 220 KB beside the circulants (B200: 227 KB per CTA, less the kernel's static shared memory)
     if (x->sp_smem > kSpMaxSmem)
         return fail(LDPC_ERR_UNSUPPORTED, "%s decoder: %d B of shared memory", dbl ? "double" : "float", x->sp_smem);
-    CUDA_TRY(allow_dynamic_smem(kfn, kSpMaxSmem));
+    x->sp_smem += edge_smem;
+    CUDA_TRY(allow_dynamic_smem(kfn, kSpMaxSmem + kSpEdgeSmem));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, x->sp_threads, x->sp_smem));
     if (per_sm < 1) return fail(LDPC_ERR_UNSUPPORTED, "float decoder: launch does not fit an SM");

@@ -52,7 +52,7 @@ constexpr int kThreads = 512;                   // __launch_bounds__ of the kern
 // The kernels are the context path's instances (sp_f32_kernel<D, P, false, 512>),
 // and a kernel's shared-memory limit is a property of the function: both
 // paths set it to the same maximum, so neither lowers it under the other.
-constexpr int kMaxSmem = ldpc::kSpMaxSmem;
+constexpr int kMaxSmem = ldpc::kSpMaxSmem;            // beside the circulants
 
 __device__ __align__(256) float g_sp_scratch[kScratchBytes / sizeof(float)];
 
@@ -92,7 +92,8 @@ int device_setup(int dev, DeviceState** out) {
         if (((uintptr_t)p & 255) != 0) return ldpc::fail(LDPC_ERR_CUDA, "scratch of device %d is not 256-byte aligned", dev);
         CUDA_TRY(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
         for (const NoallocKernel& k : kKernels)
-            CUDA_TRY(cudaFuncSetAttribute((const void*)k.k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+            CUDA_TRY(cudaFuncSetAttribute((const void*)k.k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          kMaxSmem + ldpc::kSpEdgeSmem));
         d.scratch = (float*)p;
         d.ready.store(true, std::memory_order_release);
     }
@@ -135,15 +136,16 @@ extern "C" int ldpc_decode_f32_noalloc(const ldpc_code* code, const ldpc_cfg* cf
     while (G > 1 && ((G * c.z + 31) / 32) * 32 > kThreads) --G;
     const int nstage = (c.z * c.mcol + 3) & ~3;
     auto base_bytes = [&](int g, bool stage) {
-        ldpc::fill_sp_tables(c, g, &t);
+        ldpc::fill_sp_tables(c, g, (int)sizeof(float), &t);
         return ((((size_t)g * t.stride + 3) & ~(size_t)3) + (stage ? (size_t)g * nstage : 0)) * sizeof(float);
     };
     while (G > 1 && base_bytes(G, true) > (size_t)kMaxSmem) --G;
     const bool nostage = base_bytes(G, true) > (size_t)kMaxSmem;
-    const size_t smem = base_bytes(G, !nostage);   // leaves t filled for G
+    const size_t payload = base_bytes(G, !nostage);   // leaves t filled for G
     t.nostage = nostage ? 1 : 0;
+    const size_t smem = payload + ldpc::sp_edge_bytes(t.E);
     const int threads = ((G * c.z + 31) / 32) * 32;
-    if (smem > (size_t)kMaxSmem) return fail(LDPC_ERR_UNSUPPORTED, "float decoder: %zu B of shared memory", smem);
+    if (payload > (size_t)kMaxSmem) return fail(LDPC_ERR_UNSUPPORTED, "float decoder: %zu B of shared memory", payload);
     const size_t per_cta = (size_t)t.E * threads * sizeof(float);
     if (per_cta > kScratchBytes)
         return fail(LDPC_ERR_UNSUPPORTED,

@@ -33,6 +33,7 @@ inline cudaError_t allow_dynamic_smem(const void* fn, int bytes) {
 }
 constexpr int kOmsMaxSmem = 200 * 1024;     // int8 register-shape kernels
 constexpr int kSpMaxSmem = 220 * 1024;      // float decoders (B200: 227 KB per CTA less static shared memory)
+constexpr int kSpEdgeSmem = SP_MAX_E * (int)sizeof(SpEdge);   // their circulants, beside that
 
 struct OmsLaunch {
     int max_threads, min_blocks;   // __launch_bounds__ of this compilation
@@ -172,8 +173,8 @@ inline int llr_bytes(int variant) {
            : (variant == LDPC_F64_SP || variant == LDPC_F64_OMS) ? 8 : 4;
 }
 int setup_sp(ldpc_ctx* x);
-// float-decoder tables of a code for G codewords per CTA
-void fill_sp_tables(const ldpc_code& c, int G, SpTables* t);
+// float-decoder tables of a code for G codewords per CTA, es bytes per element
+void fill_sp_tables(const ldpc_code& c, int G, int es, SpTables* t);
 int launch_sp(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s);
 int setup_gen(ldpc_ctx* x);
 int launch_gen(ldpc_ctx* x, uint64_t seed, uint64_t cw_offset, const float* snr_db, size_t n_snr, size_t n_per_snr,

@@ -61,19 +61,19 @@ __device__ __forceinline__ int32_t int_abs(int32_t q) {
 }
 
 template <int W, int DMAX>
-__device__ __forceinline__ void int_layer(const SpTables& tb, int l, int32_t* Ps, int32_t* Rt, int rstride, int t,
-                                          int gbase, int beta, int maxv) {
-    const int d = tb.rw[l], eb = tb.ebase[l], z = tb.z;
+__device__ __forceinline__ void int_layer(const SpTables& tb, int l, char* Pg, int32_t* Rt, int rstride, uint32_t tb_,
+                                          uint32_t zb, int beta, int maxv) {
+    const int d = tb.rw[l], eb = tb.ebase[l];
     int32_t q[DMAX];
-    int addr[DMAX];
+    int32_t* p[DMAX];
     int32_t mn1 = 0x7fffffff, mn2 = 0x7fffffff;
     uint32_t rx = 0;
 #pragma unroll
     for (int j = 0; j < DMAX; ++j) {
         if (j < d) {
             const int e = eb + j;
-            addr[j] = gbase + tb.colz[e] + sp_wrap(t, tb.shift[e], z);
-            const int32_t Q = int_sat<W>(Ps[addr[j]], Rt[e * rstride], true);
+            p[j] = sp_at<int32_t>(tb.edge[e], Pg, tb_, zb);
+            const int32_t Q = int_sat<W>(*p[j], Rt[e * rstride], true);
             int32_t m = int_wrap<W>(int_abs<W>(Q) - beta);
             m = m > 0 ? m : 0;
             mn2 = min(mn2, max(mn1, m));
@@ -90,7 +90,7 @@ __device__ __forceinline__ void int_layer(const SpTables& tb, int l, int32_t* Ps
             m = m > 0 ? m : 0;
             const int32_t f = m == mn1 ? f2 : f1;
             const int32_t rn = ((rx ^ (uint32_t)q[j]) & 0x80000000u) ? -f : f;
-            Ps[addr[j]] = int_sat<W>(q[j], rn, false);
+            *p[j] = int_sat<W>(q[j], rn, false);
             Rt[(eb + j) * rstride] = rn;
         }
     }
@@ -144,6 +144,8 @@ __global__ void __launch_bounds__(512) oms_int_kernel(const __grid_constant__ Sp
     // words (coalesced)
     const int rstride = RSMEM ? 1 : nthr;
     int32_t* Rt = RSMEM ? Rbase + tid * (tb.E | 1) : Rbase + tid;
+    char* const Pg = reinterpret_cast<char*>(Ps + gbase);
+    const uint32_t tb_ = 4u * (uint32_t)t, zb = 4u * (uint32_t)z;
     const TL* llr = reinterpret_cast<const TL*>(job.llr);
     const long long lo = job.ncw * blockIdx.x / gridDim.x, hi = job.ncw * (blockIdx.x + 1) / gridDim.x;
 
@@ -175,7 +177,7 @@ __global__ void __launch_bounds__(512) oms_int_kernel(const __grid_constant__ Sp
 
     for (int par = 0;; par ^= 1) {
         for (int l = 0; l < tb.L; ++l) {
-            if (active) int_layer<W, DMAX>(tb, l, Ps, Rt, rstride, t, gbase, job.beta, job.maxv);
+            if (active) int_layer<W, DMAX>(tb, l, Pg, Rt, rstride, tb_, zb, job.beta, job.maxv);
             __syncthreads();
         }
         if (tid == 0) {
@@ -191,7 +193,7 @@ __global__ void __launch_bounds__(512) oms_int_kernel(const __grid_constant__ Sp
                 uint32_t xr = 0;
                 for (int j = 0; j < d; ++j) {
                     const int e = eb + j;
-                    xr ^= (uint32_t)Ps[gbase + tb.colz[e] + sp_wrap(t, tb.shift[e], z)];
+                    xr ^= (uint32_t)*sp_at<int32_t>(tb.edge[e], Pg, tb_, zb);
                 }
                 if (xr & 0x80000000u) {
                     atomicOr(&s_synd[par], 1u << g);

@@ -5,6 +5,7 @@
 #include <utility>
 
 #include "internal.h"
+#include "sp_math.cuh"
 
 namespace ldpc {
 namespace {
@@ -216,5 +217,64 @@ extern "C" int ldpc_probe_op_rates(int device, double* ops_per_clk_sm, int n_ops
         if (names) names[op] = kOpNames[op];
     }
     cudaFree(out);
+    return LDPC_OK;
+}
+
+namespace ldpc {
+namespace {
+
+// splitmix64 (Steele, Lea, Flood, "Fast splittable pseudorandom number generators", 2014)
+__device__ uint64_t splitmix(uint64_t& s) {
+    uint64_t z = (s += 0x9E3779B97F4A7C15ull);
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+
+// A double with exponent in [lo, hi] and a random mantissa, an eighth of them with all but a few
+// bits 0 or 1 (next to a power of two, where quotients and reciprocals round hardest).
+__device__ double draw_double(uint64_t& s, int lo, int hi) {
+    uint64_t m = splitmix(s) >> 12;
+    const uint64_t q = splitmix(s);
+    if ((q & 15) == 0) m &= 15;
+    if ((q & 15) == 1) m |= 0xFFFFFFFFFFFF0ull;
+    return __longlong_as_double((long long)((uint64_t)(lo + (int)((q >> 8) % (uint64_t)(hi - lo + 1)) + 1023) << 52 | m));
+}
+
+__global__ void sp_math_kernel(int samples, unsigned long long* bad) {
+    const uint64_t id = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, all = gridDim.x * (uint64_t)blockDim.x;
+    unsigned long long n = 0;
+    for (uint64_t i = id; i <= 0x7f800000ull; i += all) {
+        const float a = __uint_as_float((uint32_t)i);
+        n += __float_as_uint(lm_tanh(__fmul_rn(a, 0.5f))) != __float_as_uint(spm_tanh_half(a));
+        if (i <= 0x3f800000ull)
+            n += __float_as_uint(__fmul_rn(2.0f, lm_atanh(a))) != __float_as_uint(spm_atanh_twice(a));
+    }
+    uint64_t s = id * 0xD1342543DE82EF95ull + 1;
+    for (int i = 0; i < samples; ++i) {
+        const double a = (i & 3) ? draw_double(s, -8, 5) : draw_double(s, -1022, 6);
+        n += __double_as_longlong(lmd_tanh(__dmul_rn(a, 0.5))) != __double_as_longlong(spm_tanh_half(a));
+        double m = (i & 1) ? 1.0 - draw_double(s, -53, -2) : draw_double(s, (i & 2) ? -6 : -1022, -1);
+        if (i == 0) m = id == 0 ? 0.0 : id == 1 ? 1.0 : m;
+        n += __double_as_longlong(__dmul_rn(2.0, lmd_atanh(m))) != __double_as_longlong(spm_atanh_twice(m));
+    }
+    if (n) atomicAdd(bad, n);
+}
+
+}  // namespace
+}  // namespace ldpc
+
+extern "C" int ldpc_probe_sp_math(int device, int samples, unsigned long long* mismatches) {
+    if (!mismatches || samples < 0) return ldpc::fail(LDPC_ERR_INVALID_ARG, "NULL result or samples < 0");
+    CUDA_TRY(cudaSetDevice(device));
+    unsigned long long* d = nullptr;
+    CUDA_TRY(cudaMalloc(&d, sizeof(*d)));
+    cudaError_t e = cudaMemset(d, 0, sizeof(*d));
+    if (e == cudaSuccess) {
+        ldpc::sp_math_kernel<<<1184, 256>>>(samples, d);
+        e = cudaMemcpy(mismatches, d, sizeof(*d), cudaMemcpyDeviceToHost);
+    }
+    cudaFree(d);
+    CUDA_TRY(e);
     return LDPC_OK;
 }

@@ -86,7 +86,7 @@ __global__ void __maxnreg__(sp_max_regs(DMAX, PROD, RSMEM)) sp_batch_kernel(cons
         job.beta = C.beta;
         job.maxv = C.maxv;
         job.r_scratch = nullptr;
-        sp_decode_range<DMAX, PROD, RSMEM>(C.t, job, ch.lo, ch.hi, sm_f,
+        sp_decode_range<DMAX, PROD, RSMEM>(C.t, C.t.edge, job, ch.lo, ch.hi, sm_f,
                                            RSMEM ? nullptr : lp.r_scratch + (long long)blockIdx.x * lp.r_words_per_cta);
     }
 }

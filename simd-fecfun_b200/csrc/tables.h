@@ -42,6 +42,14 @@ struct OmsJob {
 constexpr int SP_MAX_L = 64;
 constexpr int SP_MAX_E = 512;
 
+// One circulant as the kernels use it, in bytes of the posterior element:
+// check t's posterior in the circulant's column lies at
+// col + min_u(t + off, t + off + z), off = shift - z.
+struct SpEdge {
+    uint32_t col;                    // column * Z
+    uint32_t off;                    // shift - Z, modulo 2^32
+};
+
 struct SpTables {
     int z, mcol, n, L, G;            // G = codewords per CTA (one per group of Z threads)
     int stride;                      // posterior words per group in shared memory
@@ -50,8 +58,7 @@ struct SpTables {
     int nostage;                     // 1: no shared staging buffer; refill from global memory
     int16_t rw[SP_MAX_L];
     int16_t ebase[SP_MAX_L];         // first edge of layer l
-    int32_t colz[SP_MAX_E];          // column * Z of edge e
-    int16_t shift[SP_MAX_E];
+    SpEdge edge[SP_MAX_E];
 };
 
 template <class T>                   // T = float or double

@@ -58,7 +58,14 @@ struct TrainJob {
 
 constexpr int TRAIN_MAX_ITERS = 64;
 
-__device__ __forceinline__ int tr_wrap(int t, int s, int z) { return (int)min((unsigned)(t + s), (unsigned)(t + s - z)); }
+// byte offset of check t's posterior in circulant e's column
+__device__ __forceinline__ uint32_t tr_pos(SpEdge e, int t, int z) {
+    const uint32_t w = 4u * (uint32_t)t + e.off;
+    return e.col + min(w, w + 4u * (uint32_t)z);
+}
+__device__ __forceinline__ float& tr_at(float* P, uint32_t pos) {
+    return *reinterpret_cast<float*>(reinterpret_cast<char*>(P) + pos);
+}
 
 // One layer's forward update for check row t; if keep_q, Q replaces the
 // message in R (the backward recompute).
@@ -67,7 +74,7 @@ __device__ __forceinline__ void tr_layer(const SpTables& tb, int l, float* P, fl
                                          bool keep_q) {
     const int d = tb.rw[l], eb = tb.ebase[l], z = tb.z;
     float q[DMAX];
-    int addr[DMAX];
+    uint32_t pos[DMAX];
     float mn1 = __int_as_float(0x7f800000), mn2 = mn1;
     int idx = 0;
     uint32_t rx = 0;
@@ -75,8 +82,8 @@ __device__ __forceinline__ void tr_layer(const SpTables& tb, int l, float* P, fl
     for (int j = 0; j < DMAX; ++j) {
         if (j < d) {
             const int e = eb + j;
-            addr[j] = tb.colz[e] + tr_wrap(t, tb.shift[e], z);
-            const float Q = __fsub_rn(P[addr[j]], R[e * z + t]);
+            pos[j] = tr_pos(tb.edge[e], t, z);
+            const float Q = __fsub_rn(tr_at(P, pos[j]), R[e * z + t]);
             float a = __fsub_rn(fabsf(Q), beta);
             a = a > 0.0f ? a : 0.0f;
             if (a < mn1) {
@@ -97,7 +104,7 @@ __device__ __forceinline__ void tr_layer(const SpTables& tb, int l, float* P, fl
             f = maxv < f ? maxv : f;
             const uint32_t sg = (rx ^ __float_as_uint(q[j])) & 0x80000000u;
             const float rn = __uint_as_float(__float_as_uint(f) ^ sg);
-            P[addr[j]] = __fadd_rn(q[j], rn);
+            tr_at(P, pos[j]) = __fadd_rn(q[j], rn);
             R[(eb + j) * z + t] = keep_q ? q[j] : rn;
         }
     }
@@ -109,7 +116,7 @@ __device__ __forceinline__ bool tr_syndrome_ok(const SpTables& tb, const float* 
         uint32_t x = 0;
         for (int j = 0; j < tb.rw[l]; ++j) {
             const int e = tb.ebase[l] + j;
-            x ^= __float_as_uint(P[tb.colz[e] + tr_wrap(t, tb.shift[e], tb.z)]);
+            x ^= __float_as_uint(tr_at(const_cast<float*>(P), tr_pos(tb.edge[e], t, tb.z)));
         }
         ok = !(x & 0x80000000u);
     }
@@ -255,7 +262,7 @@ __global__ void __launch_bounds__(512) oms_train_bwd(const __grid_constant__ SpT
                 if (active) {
                     const int d = tb.rw[l], eb = tb.ebase[l];
                     float q[DMAX], a[DMAX], gq[DMAX], gf[DMAX];
-                    int addr[DMAX];
+                    uint32_t pos[DMAX];
                     float mn1 = __int_as_float(0x7f800000), mn2 = mn1;
                     int i1 = 0, i2 = -1;
                     uint32_t rx = 0;
@@ -263,7 +270,7 @@ __global__ void __launch_bounds__(512) oms_train_bwd(const __grid_constant__ SpT
                     for (int j = 0; j < DMAX; ++j) {
                         if (j < d) {
                             const int e = eb + j;
-                            addr[j] = tb.colz[e] + tr_wrap(t, tb.shift[e], z);
+                            pos[j] = tr_pos(tb.edge[e], t, z);
                             q[j] = QR[e * z + t];
                             a[j] = __fsub_rn(fabsf(q[j]), beta);
                             const float m = a[j] > 0.0f ? a[j] : 0.0f;
@@ -284,7 +291,7 @@ __global__ void __launch_bounds__(512) oms_train_bwd(const __grid_constant__ SpT
                     for (int j = 0; j < DMAX; ++j) {
                         if (j < d) {
                             const int e = eb + j;
-                            const float gpost = gP[addr[j]];
+                            const float gpost = tr_at(gP, pos[j]);
                             const float grn = gpost + gR[e * z + t];
                             const float fu = j == i1 ? mn2 : mn1;
                             const bool neg = ((rx ^ __float_as_uint(q[j])) & 0x80000000u) != 0;
@@ -301,7 +308,7 @@ __global__ void __launch_bounds__(512) oms_train_bwd(const __grid_constant__ SpT
                             const float ga = a[j] > 0.0f ? gm : 0.0f;
                             gb -= ga;
                             gq[j] += q[j] < 0.0f ? -ga : ga;
-                            gP[addr[j]] = gq[j];
+                            tr_at(gP, pos[j]) = gq[j];
                             gR[(eb + j) * z + t] = -gq[j];
                         }
                     }

@@ -37,11 +37,12 @@ def generate(path):
             out.append("    out[%d] = n[%d];" % (j, k))
         out.append("}")
         out.append("")
-    out.append("template <int DMAX, class T, class Comb, class Clamp>")
+    out.append("// the tree of weight d, LO <= d <= HI")
+    out.append("template <int LO, int HI, class T, class Comb, class Clamp>")
     out.append("__device__ __forceinline__ void run_tree(int d, T* x, T* out, Comb comb, Clamp clamp) {")
     out.append("    switch (d) {")
     for d in range(2, MAX_D + 1):
-        out.append("        case %d: if constexpr (DMAX >= %d) tree_%d(x, out, comb, clamp); break;" % (d, d, d))
+        out.append("        case %d: if constexpr (LO <= %d && %d <= HI) tree_%d(x, out, comb, clamp); break;" % (d, d, d, d))
     out.append("        default: break;")
     out.append("    }")
     out.append("}")

@@ -99,6 +99,7 @@ _PROTOS = {
     "ldpc_probe_int32_peak": (C.c_int, [C.c_int, C.POINTER(C.c_double)]),
     "ldpc_probe_fp32_peak": (C.c_int, [C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "ldpc_probe_op_rates": (C.c_int, [C.c_int, C.POINTER(C.c_double), C.c_int, C.POINTER(C.c_char_p)]),
+    "ldpc_probe_sp_math": (C.c_int, [C.c_int, C.c_int, C.POINTER(C.c_ulonglong)]),
     "ldpc_decode_f32_noalloc": (C.c_int, [_vp, C.POINTER(Cfg), _vp, _sz, _vp, _vp, _vp, _vp]),
     "ldpc_batch_create": (C.c_int, [C.POINTER(_vp), C.POINTER(Cfg), C.c_int, C.c_int, C.POINTER(_vp)]),
     "ldpc_batch_set_offsets": (C.c_int, [_vp, C.c_int, _vp]),
@@ -161,6 +162,13 @@ def probe_op_rates(device: int = 0):
     names = (C.c_char_p * n)()
     check(lib.ldpc_probe_op_rates(device, v, n, names))
     return [(names[i].decode(), v[i]) for i in range(n)]
+
+
+def probe_sp_math(device: int = 0, samples: int = 1000) -> int:
+    """Results of the branch-free tanh/atanh that differ from the shared functions."""
+    v = C.c_ulonglong()
+    check(lib.ldpc_probe_sp_math(device, samples, C.byref(v)))
+    return v.value
 
 
 def _ptr(x) -> Optional[int]:
