@@ -294,6 +294,19 @@ int ldpc_learned_forward(ldpc_ctx *ctx, const float *llr, size_t n, int iters, c
 int ldpc_learned_backward(ldpc_ctx *ctx, size_t n, int iters, const float *beta, const float *ckpt_p,
                           const float *ckpt_r, const uint8_t *cw_bits, const float *loss_w, float inv_norm,
                           float *gbeta_part, float *grad_llr, void *stream);
+/* The loss above and its gradient in one launch, without checkpoints in
+ * caller memory: what LearnedOMSLoss runs.  ldpc_learned_loss_size gives the
+ * number of partial losses and partial gradients and the scratch needed for
+ * want_grad != 0.  loss_part [loss_rows] (double; their sum is L), gbeta_part
+ * [grad_rows][iters*mrow] (column sums = dL/dbeta) and scratch
+ * [scratch_floats]; gbeta_part = scratch = NULL: the loss alone.  All partial
+ * sums are in a fixed order.  Takes the codes that ldpc_learned_backward
+ * (with the gradient) or ldpc_learned_forward (without) takes. */
+int ldpc_learned_loss_size(ldpc_ctx *ctx, size_t n, int iters, int want_grad, int *loss_rows, int *grad_rows,
+                           size_t *scratch_floats);
+int ldpc_learned_loss(ldpc_ctx *ctx, const float *llr, const uint8_t *cw_bits, size_t n, int iters,
+                      const float *beta, const float *loss_w, float inv_norm, float *scratch, float *gbeta_part,
+                      double *loss_part, void *stream);
 /* Decoding with learned offsets: up to `iters` iterations with early exit on
  * the syndrome, as the float decoders do; outputs as ldpc_decode_f32. */
 int ldpc_learned_decode(ldpc_ctx *ctx, const float *llr, size_t n, int iters, const float *beta, float *post_out,

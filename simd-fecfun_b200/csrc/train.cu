@@ -5,6 +5,7 @@
 
 #include "internal.h"
 #include "train.cuh"
+#include "train_step.cuh"
 
 using ldpc::fail;
 
@@ -53,6 +54,51 @@ int geometry(ldpc_ctx* x, size_t n, bool backward, Geometry* g) {
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)g->k, g->threads, g->smem));
     if (per_sm < 1) return fail(LDPC_ERR_UNSUPPORTED, "learned decoder: launch does not fit an SM");
     g->grid = (int)std::max<long long>(1, std::min<long long>((long long)n, (long long)per_sm * x->sms));
+    return LDPC_OK;
+}
+
+// Loss (and gradient) kernel: codewords per CTA as the float decoders choose
+// them, fewer while the CTA's shared memory is above what lets five share an SM.
+typedef void (*step_fn)(const ldpc::SpTables, const ldpc::TrainStepJob);
+struct StepKernels {
+    int dmax, nt;
+    step_fn grad, loss;
+};
+#define TSK(D_, N_) {D_, N_, ldpc::oms_train_step<D_, N_, true>, ldpc::oms_train_step<D_, N_, false>}
+const StepKernels kStep[] = {TSK(8, 128), TSK(16, 128), TSK(32, 128), TSK(8, 512), TSK(16, 512), TSK(32, 512)};
+#undef TSK
+
+struct StepGeometry {
+    step_fn k;
+    int threads, smem, grid, nt;
+    ldpc::SpTables t;
+};
+
+int step_geometry(ldpc_ctx* x, size_t n, int iters, bool grad, StepGeometry* g) {
+    Geometry unused;
+    // the codes that the separate forward and adjoint kernels take
+    if (int rc = geometry(x, n, grad, &unused)) return rc;
+    const ldpc_code& c = x->code;
+    int G = std::max(1, std::min(32, 128 / c.z));
+    auto smem = [&](int k) {
+        ldpc::fill_sp_tables(c, k, (int)sizeof(float), &g->t);
+        return ldpc::train_step_smem(k, g->t.stride, g->t.E, g->t.mcol, ((k * c.z + 31) / 32) * 32, iters * g->t.L);
+    };
+    while (G > 1 && smem(G) > 45 * 1024) --G;
+    g->smem = smem(G);
+    g->threads = ((G * c.z + 31) / 32) * 32;
+    g->nt = g->threads <= 128 ? 128 : 512;
+    g->k = nullptr;
+    for (const StepKernels& k : kStep)
+        if (!g->k && k.nt == g->nt && c.max_row_weight <= k.dmax) g->k = grad ? k.grad : k.loss;
+    if (g->smem > kTrainMaxSmem)
+        return fail(LDPC_ERR_UNSUPPORTED, "learned decoder: %d B of shared memory per codeword", g->smem);
+    CUDA_TRY(ldpc::allow_dynamic_smem((const void*)g->k, kTrainMaxSmem));
+    int per_sm = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)g->k, g->threads, g->smem));
+    if (per_sm < 1) return fail(LDPC_ERR_UNSUPPORTED, "learned decoder: launch does not fit an SM");
+    const long long want = ((long long)n + G - 1) / G;
+    g->grid = (int)std::max<long long>(1, std::min<long long>(want, (long long)per_sm * x->sms));
     return LDPC_OK;
 }
 
@@ -119,6 +165,44 @@ int ldpc_learned_backward(ldpc_ctx* x, size_t n, int iters, const float* beta, c
     j.gbeta_part = gbeta_part;
     j.grad_llr = grad_llr;
     g.k<<<g.grid, g.threads, g.smem, (cudaStream_t)stream>>>(x->spt, j);
+    CUDA_TRY(cudaGetLastError());
+    return LDPC_OK;
+}
+
+int ldpc_learned_loss_size(ldpc_ctx* x, size_t n, int iters, int want_grad, int* loss_rows, int* grad_rows,
+                           size_t* scratch_floats) {
+    if (int rc = check_iters(iters)) return rc;
+    StepGeometry g;
+    if (int rc = step_geometry(x, n, iters, want_grad != 0, &g)) return rc;
+    if (loss_rows) *loss_rows = g.grid;
+    if (grad_rows) *grad_rows = g.grid * (g.threads / 32);
+    if (scratch_floats) *scratch_floats = (size_t)g.grid * iters * (g.t.E + g.t.mcol) * g.nt;
+    return LDPC_OK;
+}
+
+int ldpc_learned_loss(ldpc_ctx* x, const float* llr, const uint8_t* cw_bits, size_t n, int iters, const float* beta,
+                      const float* loss_w, float inv_norm, float* scratch, float* gbeta_part, double* loss_part,
+                      void* stream) {
+    if (int rc = check_iters(iters)) return rc;
+    if (!loss_part || (n && (!llr || !cw_bits || !beta || !loss_w)) || (!scratch != !gbeta_part))
+        return fail(LDPC_ERR_INVALID_ARG, "NULL buffer");
+    StepGeometry g;
+    if (int rc = step_geometry(x, n, iters, scratch != nullptr, &g)) return rc;
+    CUDA_TRY(cudaSetDevice(x->device));
+    ldpc::TrainStepJob j;
+    memset(&j, 0, sizeof(j));
+    j.llr = llr;
+    j.cw_bits = cw_bits;
+    j.ncw = (long long)n;
+    j.iters = iters;
+    j.beta = beta;
+    j.loss_w = loss_w;
+    j.maxv = x->maxf;
+    j.inv_norm = inv_norm;
+    j.scratch = scratch;
+    j.gbeta_part = gbeta_part;
+    j.loss_part = loss_part;
+    g.k<<<g.grid, g.threads, g.smem, (cudaStream_t)stream>>>(g.t, j);
     CUDA_TRY(cudaGetLastError());
     return LDPC_OK;
 }

@@ -1,8 +1,8 @@
 """Learned offsets for layered offset min-sum.
 
-* :class:`LearnedOMSLoss` -- ``torch.autograd.Function`` over the CUDA
-  forward (per-iteration checkpoints) and hand-written adjoint kernels
-  (``ldpc_learned_forward`` / ``ldpc_learned_backward``).
+* :class:`LearnedOMSLoss` -- ``torch.autograd.Function`` over one CUDA kernel
+  that unrolls the decoder, evaluates the loss and runs the hand-written
+  adjoint (``ldpc_learned_loss``).
 * :func:`reference_loss` -- the same unrolled decoder and loss written with
   differentiable torch operations (any dtype, CPU or GPU): the reference
   gradient for the adjoint, and the function the finite-difference checks
@@ -46,37 +46,39 @@ class LearnedOMSLoss(torch.autograd.Function):
 
     @staticmethod
     def forward(fctx, beta, llr, cw_bits, loss_w, ctx):
-        iters = beta.shape[0]
+        iters, L = beta.shape
         n, N = llr.shape
-        E = ctx.info.edges
+        grad = fctx.needs_input_grad[0]
         beta = beta.detach().contiguous().float()
         llr = llr.contiguous().float()
-        ckpt_p = torch.empty((iters + 1, n, N), dtype=torch.float32, device=llr.device)
-        ckpt_r = torch.empty((iters, n, E), dtype=torch.float32, device=llr.device)
-        capi.check(capi.lib.ldpc_learned_forward(ctx.h, llr.data_ptr(), n, iters, beta.data_ptr(), ckpt_p.data_ptr(),
-                                                 ckpt_r.data_ptr(), _stream()))
-        s = 1.0 - 2.0 * cw_bits.float()
-        per_it = F.softplus(-s.unsqueeze(0) * ckpt_p[1:]).sum(dim=(1, 2))
-        loss = (loss_w.float() * per_it).sum() / float(n * N)
-        fctx.save_for_backward(beta, ckpt_p, ckpt_r, cw_bits.contiguous(), loss_w.contiguous().float())
-        fctx.ctx = ctx
-        fctx.shape = (n, N)
-        return loss
+        cw_bits = cw_bits.expand(n, N).contiguous()
+        if cw_bits.dtype not in (torch.uint8, torch.bool):
+            cw_bits = cw_bits.to(torch.uint8)
+        loss_w = (loss_w if loss_w.dim() else loss_w.to(llr.device)).float().expand(iters).contiguous()
+        for t in (beta, llr, cw_bits, loss_w):
+            if not t.is_cuda or t.device != llr.device:
+                raise RuntimeError("LearnedOMSLoss needs its tensors on one CUDA device")
+        inv_norm = 1.0 / float(n * N) if n * N else float("nan")
+        rows, grows, words = C.c_int(), C.c_int(), C.c_size_t()
+        capi.check(capi.lib.ldpc_learned_loss_size(ctx.h, n, iters, int(grad), C.byref(rows), C.byref(grows),
+                                                   C.byref(words)))
+        loss = torch.empty(rows.value, dtype=torch.float64, device=llr.device)
+        part = scratch = None
+        if grad:
+            part = torch.empty((grows.value, iters * L), dtype=torch.float32, device=llr.device)
+            scratch = torch.empty(words.value, dtype=torch.float32, device=llr.device)
+        capi.check(capi.lib.ldpc_learned_loss(ctx.h, llr.data_ptr(), cw_bits.data_ptr(), n, iters, beta.data_ptr(),
+                                              loss_w.data_ptr(), inv_norm, capi._ptr(scratch), capi._ptr(part),
+                                              loss.data_ptr(), _stream()))
+        # the gradient is at hand already; the inputs are saved so that autograd
+        # still sees one changed in place before backward
+        fctx.save_for_backward(beta, cw_bits, loss_w, part.sum(dim=0).view(iters, L) if grad else None)
+        return loss.sum().float()
 
     @staticmethod
     def backward(fctx, g):
-        beta, ckpt_p, ckpt_r, cw_bits, loss_w = fctx.saved_tensors
-        ctx = fctx.ctx
-        n, N = fctx.shape
-        iters, L = beta.shape
-        grid = C.c_int()
-        capi.check(capi.lib.ldpc_learned_grid(ctx.h, n, C.byref(grid)))
-        part = torch.empty((grid.value, iters * L), dtype=torch.float32, device=beta.device)
-        capi.check(capi.lib.ldpc_learned_backward(ctx.h, n, iters, beta.data_ptr(), ckpt_p.data_ptr(), ckpt_r.data_ptr(),
-                                                  cw_bits.data_ptr(), loss_w.data_ptr(), 1.0 / float(n * N),
-                                                  part.data_ptr(), None, _stream()))
-        gbeta = part.sum(dim=0).view(iters, L) * g
-        return gbeta, None, None, None, None
+        gbeta = fctx.saved_tensors[3]
+        return gbeta * g if gbeta is not None else None, None, None, None, None
 
 
 def layer_tables(code):

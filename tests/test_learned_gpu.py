@@ -159,3 +159,46 @@ def test_training_lowers_the_loss(capi):
     assert l1 < 0.98 * l0
     cwer, ber, avg_it = learned.evaluate(ctx, code, beta, learned.snr_from_ebn0(2.0, 0.5), 4096)
     assert 0.0 <= cwer < 0.5 and 1.0 <= avg_it <= 6.0
+
+
+@pytest.mark.parametrize("name,z,n", [("16e 1/2", 24, 7), ("16e 1/2", 24, 5), ("16e 1/2", 96, 3), ("16e 1/2", 192, 2),
+                                      ("11n 3/4 z27", None, 11), ("16e 5/6", 24, 9), ("5GNR_n1600_k320", None, 5)])
+def test_loss_kernel_matches_checkpointed_kernels(capi, name, z, n):
+    """The one-launch loss and gradient against the checkpointing forward and
+    adjoint kernels: several codewords per CTA with a ragged last group,
+    CTAs above 128 threads, rows up to weight 20, more than 32 columns.  The
+    forward values are the same; the sums differ in order and in the
+    logistic's last bits (n x N terms of ~1e-7 relative error: 1e-5 allowed)."""
+    import ctypes as C
+    import torch
+    import torch.nn.functional as F
+    from ldpc_b200 import codes, learned
+    code = codes.make_code(name, z_over=z) if z else codes.code_by_name(name)
+    ctx = capi.Context(capi.Code.from_tables(code), variant=capi.LDPC_F32_OMS, max_iter=10, max_row_metric=5.0, beta=0.5,
+                       llr_scale=1.0, max_abs_llr=1e9)
+    iters, N, L = 3, code.n, code.mrow
+    g = torch.Generator(device="cuda").manual_seed(n)
+    llr = 2.0 + 3.0 * torch.randn((n, N), generator=g, device="cuda")
+    bits = (torch.rand((n, N), generator=g, device="cuda") < 0.1).to(torch.uint8)
+    beta = (0.5 + 0.1 * torch.randn((iters, L), generator=g, device="cuda")).requires_grad_(True)
+    w = torch.tensor([1.0, 0.5, 2.0], device="cuda")
+    loss = learned.LearnedOMSLoss.apply(beta, llr, bits, w, ctx)
+    loss.backward()
+    with torch.no_grad():
+        alone = learned.LearnedOMSLoss.apply(beta.detach(), llr, bits, w, ctx)
+    assert alone.item() == loss.item()
+    ckpt_p = torch.empty((iters + 1, n, N), device="cuda")
+    ckpt_r = torch.empty((iters, n, ctx.info.edges), device="cuda")
+    b = beta.detach()
+    capi.check(capi.lib.ldpc_learned_forward(ctx.h, llr.data_ptr(), n, iters, b.data_ptr(), ckpt_p.data_ptr(),
+                                             ckpt_r.data_ptr(), None))
+    s = 1.0 - 2.0 * bits.double()
+    want = (w.double() * F.softplus(-s * ckpt_p[1:].double()).sum(dim=(1, 2))).sum() / (n * N)
+    grid = C.c_int()
+    capi.check(capi.lib.ldpc_learned_grid(ctx.h, n, C.byref(grid)))
+    part = torch.empty((grid.value, iters * L), device="cuda")
+    capi.check(capi.lib.ldpc_learned_backward(ctx.h, n, iters, b.data_ptr(), ckpt_p.data_ptr(), ckpt_r.data_ptr(),
+                                              bits.data_ptr(), w.data_ptr(), 1.0 / (n * N), part.data_ptr(), None, None))
+    ref = part.double().sum(dim=0).view(iters, L)
+    assert abs(loss.item() - want.item()) <= 1e-6 * want.item()
+    assert (beta.grad.double() - ref).norm() <= 1e-5 * ref.norm()
