@@ -270,8 +270,9 @@ int float_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int thread
 
 // One persistent launch of the run-time-table int8 kernel over the jobs; its
 // kernel variant, shared memory and message placement come from the codes
-// the jobs use.
-int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads, int cpc, ldpc_batch_plan** out) {
+// the jobs use.  share: the jobs' part of the work that runs beside them.
+int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads, int cpc, double share,
+              ldpc_batch_plan** out) {
     const int nc = (int)b->codes.size();
     std::vector<char> used(nc, 0);
     for (int i = 0; i < n_jobs; ++i) used[jobs[i].code] = 1;
@@ -282,7 +283,7 @@ int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads
         if (!used[c]) continue;
         const ldpc_code& cd = b->codes[c];
         const int n = cd.z * cd.mcol, E = (int)cd.row_cols.size();
-        G[c] = std::max(1, std::min(16, threads / cd.z));
+        G[c] = std::max(1, std::min(ldpc::kRtMaxG, threads / cd.z));
         while (G[c] > 1 && ldpc::rt_smem_bytes(n, G[c], E, 0, false) > (size_t)ldpc::kRtMaxSmem) --G[c];
         if (ldpc::rt_smem_bytes(n, G[c], E, 0, false) > (size_t)ldpc::kRtMaxSmem)
             return fail(LDPC_ERR_UNSUPPORTED, "batch plan: code %d (N=%d) does not fit shared memory", c, n);
@@ -352,11 +353,28 @@ int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads
         j.code = s.code;
         const ldpc_code& cd = b->codes[s.code];
         cost[i] = (long long)cd.row_cols.size() * cd.z;
-        minc[i] = 8 * G[s.code];     // a chunk keeps its 2G slots busy for a while
     }
     std::vector<ldpc::RtChunk> chunks;
     std::vector<long long> ncw(n_jobs);
     for (int i = 0; i < n_jobs; ++i) ncw[i] = hj[i].ncw;
+    // codewords per word: rounds of codewords over the plan's quads, each code's
+    // weighted by its share of the work
+    double cws = 0, work = 0, gw = 0;
+    for (int i = 0; i < n_jobs; ++i) {
+        cws += (double)ncw[i];
+        work += (double)ncw[i] * (double)cost[i];
+        gw += (double)ncw[i] * (double)cost[i] * G[jobs[i].code];
+    }
+    const int half = work > 0 ? ldpc::rt_half(cws, gw / work * (double)ctas * share) : 0;
+    // smallest chunk: one round of a CTA's slots (fewer when there are not enough codewords for the
+    // plan's share of the CTAs), two rounds for large plans.  18 802.11 codes in 13 launches side by
+    // side: 1000 codewords each 1.08 -> 0.88 ms, 3000 each 2.47 -> 1.73 ms against a minimum of four
+    // rounds; 10000 each 4.9 ms with two rounds, 5.3 ms with one
+    const double per_cta = cws / ((double)ctas * share);
+    for (int i = 0; i < n_jobs; ++i) {
+        const double round = (half ? 2.0 : 4.0) * G[jobs[i].code];
+        minc[i] = std::max(1, (int)(per_cta >= 150 ? 2 * round : std::min(round, per_cta)));
+    }
     make_chunks(ncw, cost, minc, ctas * cpc, chunks);
     const int n_chunks = (int)chunks.size();
     p->grid = (int)std::max(1LL, std::min<long long>(ctas, n_chunks));
@@ -384,6 +402,7 @@ int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads
     p->lp.r_words_per_cta = words;
     CUDA_TRY(cudaMalloc(&p->d_claim, sizeof(unsigned int)));
     p->lp.claim = p->d_claim;
+    p->lp.half = half;
     if (!p->d_jobs) p->lp.n_chunks = 0;
     p->n_chunks = p->lp.n_chunks;
     *out = p.release();
@@ -403,7 +422,7 @@ struct PlanClass {
 int int8_class(const ldpc_batch* b, int c, int threads, PlanClass* out) {
     const ldpc_code& cd = b->codes[c];
     const int n = cd.z * cd.mcol, E = (int)cd.row_cols.size();
-    int G = std::max(1, std::min(16, threads / cd.z));
+    int G = std::max(1, std::min(ldpc::kRtMaxG, threads / cd.z));
     while (G > 1 && ldpc::rt_smem_bytes(n, G, E, 0, false) > (size_t)ldpc::kRtMaxSmem) --G;
     const bool rsmem = ldpc::rt_smem_bytes(n, G, E, threads, true) <= (size_t)ldpc::kRtMaxSmem;
     bool quirk = false;
@@ -423,7 +442,7 @@ int int8_class(const ldpc_batch* b, int c, int threads, PlanClass* out) {
     return LDPC_OK;
 }
 
-// A code's own CTA width, the single-code context's: int8 G pairs of Z rows
+// A code's own CTA width, the single-code context's: int8 G quads of Z rows
 // (rt_default_G: at most 128 threads, 256 for N > 2048, fewest idle lanes),
 // float G = 128 / Z codewords per CTA; G*Z rounded to 32.
 int default_width(const ldpc_batch* b, int c) {
@@ -482,8 +501,9 @@ std::vector<ldpc_batch_job> class_jobs(const ldpc_batch* b, const ldpc_batch_job
     return sub;
 }
 
-int one_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads, int cpc, ldpc_batch_plan** out) {
-    return b->variant == LDPC_INT8_OMS ? int8_plan(b, jobs, n_jobs, threads, cpc, out)
+int one_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads, int cpc, double share,
+             ldpc_batch_plan** out) {
+    return b->variant == LDPC_INT8_OMS ? int8_plan(b, jobs, n_jobs, threads, cpc, share, out)
                                        : float_plan(b, jobs, n_jobs, threads, cpc, out);
 }
 
@@ -494,14 +514,20 @@ int one_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads,
 // codes' own width and `cpc`.
 int plans_by_class(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, bool explicit_threads, int threads,
                    int cpc, ldpc_batch_plan** out) {
-    if (getenv("LDPC_BATCH_ONE_LAUNCH") || n_jobs < 2) return one_plan(b, jobs, n_jobs, threads, cpc, out);
+    if (getenv("LDPC_BATCH_ONE_LAUNCH") || n_jobs < 2) return one_plan(b, jobs, n_jobs, threads, cpc, 1.0, out);
     std::vector<int> code_cls, cls_threads;
     int n_cls = 0;
     if (int rc = plan_classes(b, jobs, n_jobs, explicit_threads, threads, code_cls, cls_threads, &n_cls)) return rc;
     if (n_cls < 2) {
         if (!explicit_threads && n_cls == 1) threads = cls_threads[0];
-        return one_plan(b, jobs, n_jobs, threads, cpc, out);
+        return one_plan(b, jobs, n_jobs, threads, cpc, 1.0, out);
     }
+    auto work = [b](const ldpc_batch_job* j, size_t n) {
+        double w = 0;
+        for (size_t i = 0; i < n; ++i) w += (double)j[i].n * (double)b->codes[j[i].code].row_cols.size() * b->codes[j[i].code].z;
+        return w;
+    };
+    const double total = std::max(1.0, work(jobs, (size_t)n_jobs));
     std::unique_ptr<ldpc_batch_plan, PlanDel> p(new ldpc_batch_plan);
     p->device = b->device;
     for (int k = 0; k < n_cls; ++k) {
@@ -514,7 +540,7 @@ int plans_by_class(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, bool e
             c = b->code_cpc[sub[0].code];
         }
         ldpc_batch_plan* part = nullptr;
-        if (int rc = one_plan(b, sub.data(), (int)sub.size(), t, c, &part)) return rc;
+        if (int rc = one_plan(b, sub.data(), (int)sub.size(), t, c, std::max(1e-3, work(sub.data(), sub.size()) / total), &part)) return rc;
         p->parts.push_back(part);
         p->n_chunks += part->n_chunks;
     }

@@ -1,6 +1,7 @@
 // Host side of the int8 offset min-sum decoder over run-time code tables:
 // code description, launch geometry, single-code launch.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
@@ -35,17 +36,31 @@ int rt_stride(int n, int G) {
     return n + (((spread - n) % 32) + 32) % 32;
 }
 
-size_t rt_smem_bytes(int n, int G, int E, int threads, bool rsmem) {
+// tables, posteriors and staging of G quads
+static size_t rt_base_bytes(int n, int G, int E, bool stage) {
     const size_t nstage = (size_t)((n + 15) & ~15);
-    return (size_t)rt_code_bytes() + (((size_t)G * rt_stride(n, G) * 4 + 15) & ~(size_t)15) + 2 * (size_t)G * nstage +
-           (rsmem ? (size_t)(E | 1) * threads * 4 : 0);   // odd per-thread stride
+    return (size_t)rt_code_bytes(E) + (((size_t)G * rt_stride(n, G) * 4 + 15) & ~(size_t)15) +
+           (stage ? 4 * (size_t)G * nstage : 0);
+}
+
+bool rt_nostage(int n, int G, int E) { return rt_base_bytes(n, G, E, true) > (size_t)kRtMaxSmem; }
+
+// A row of four codewords takes about 1.35 times as long as a row of two (802.11n
+// 2/3 Z = 81, one round of codewords: 90 against 67 us; 5G NR base graph 1: 0.98
+// against 0.70 ms), so four per word pay as soon as they save rounds.  Two per
+// word up to four rounds lost: 3000 codewords of the former 192 against 171 us,
+// 500 of the latter 1.02 against 0.83 ms.
+int rt_half(double n, double quads) { return std::ceil(n / (2 * quads)) < 1.35 * std::ceil(n / (4 * quads)) ? 1 : 0; }
+
+size_t rt_smem_bytes(int n, int G, int E, int threads, bool rsmem) {
+    return rt_base_bytes(n, G, E, !rt_nostage(n, G, E)) + (rsmem ? (size_t)(E | 1) * threads * 4 : 0);   // odd per-thread stride
 }
 
 int rt_default_G(int z, int n) {
     const int cap = n <= 2048 ? 128 : 256;
     int G = 1;
     double best = 0.0;
-    for (int g = 1; g <= 16 && g * z <= cap; ++g) {
+    for (int g = 1; g <= kRtMaxG && g * z <= cap; ++g) {
         const double eff = (double)(g * z) / (((g * z + 31) / 32) * 32);
         if (eff >= best - 1e-9) {
             best = eff;
@@ -64,7 +79,7 @@ int make_rt_code(const ldpc_code& c, int max_iter, uint32_t maxv2, const int* be
                     RT_MAX_E);
     if (c.z > RT_MAX_Z) return fail(LDPC_ERR_UNSUPPORTED, "int8 decoder: Z=%d > %d", c.z, RT_MAX_Z);
     if (!rt_dmax(c.max_row_weight)) return fail(LDPC_ERR_UNSUPPORTED, "int8 decoder: row weight %d > 32", c.max_row_weight);
-    if (G < 1 || G > 16) return fail(LDPC_ERR_INVALID_ARG, "int8 decoder: %d codeword pairs per CTA", G);
+    if (G < 1 || G > kRtMaxG) return fail(LDPC_ERR_INVALID_ARG, "int8 decoder: %d codeword quads per CTA", G);
     RtCode& r = *out;
     memset(&r, 0, sizeof(r));
     r.z = c.z;
@@ -73,6 +88,7 @@ int make_rt_code(const ldpc_code& c, int max_iter, uint32_t maxv2, const int* be
     r.E = E;
     r.G = G;
     r.stride = rt_stride(r.n, G);
+    r.nostage = rt_nostage(r.n, G, E) ? 1 : 0;
     r.kbits = c.z * (c.mcol - c.mrow);
     r.hard_words = (r.kbits + 31) / 32;
     r.num_par = c.num_par;
@@ -88,7 +104,10 @@ int make_rt_code(const ldpc_code& c, int max_iter, uint32_t maxv2, const int* be
         r.ebase[l] = (int16_t)e0;
         e0 += c.row_weights[l];
     }
-    for (int e = 0; e < E; ++e) r.edge[e] = ((uint32_t)(c.row_cols[e] * c.z) << 9) | (uint32_t)c.row_shifts[e];
+    for (int l = c.mrow - 1; l >= 0; --l)
+        r.run[l] = l + 1 < c.mrow && r.rw[l + 1] == r.rw[l] ? r.run[l + 1] : (int16_t)(l + 1);
+    for (int e = 0; e < E; ++e)
+        r.edge[e] = {4u * (uint32_t)(c.row_cols[e] * c.z), 4u * (uint32_t)(c.row_shifts[e] - c.z)};
     return LDPC_OK;
 }
 
@@ -103,7 +122,7 @@ int setup_oms_rt(ldpc_ctx* x) {
     for (int v : x->layer_beta8) quirk |= v == 0;
     for (int v : x->tab_beta8) quirk |= v == 0;
     const bool force_global = getenv("LDPC_OMS_RT_GLOBAL") != nullptr;
-    // Codeword pairs per CTA (LDPC_OMS_G overrides): CTAs of at most 128
+    // Quads of codewords per CTA (LDPC_OMS_G overrides): CTAs of at most 128
     // threads for codes of N <= 2048 (short barriers, several CTAs per SM),
     // 256 for longer ones, and of those the G whose G Z rows leave the fewest
     // of the CTA's lanes idle (the larger G on a tie; G = 1 when Z exceeds the
@@ -112,7 +131,7 @@ int setup_oms_rt(ldpc_ctx* x) {
     // of it; the former ~256-thread default for every code lost up to 35 % on
     // the short ones, a 128-thread cap up to 41 % on 5G NR base graph 2.
     int G = rt_default_G(c.z, n);
-    if (const char* e = getenv("LDPC_OMS_G")) G = std::max(1, std::min(16, atoi(e)));
+    if (const char* e = getenv("LDPC_OMS_G")) G = std::max(1, std::min(kRtMaxG, atoi(e)));
     while (G > 1 && ((G * c.z + 31) / 32) * 32 > kRtMaxThreads) --G;
     while (G > 1 && rt_smem_bytes(n, G, E, 0, false) > (size_t)kRtMaxSmem) --G;
     const int threads = ((G * c.z + 31) / 32) * 32;
@@ -171,8 +190,10 @@ int launch_oms_rt(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     j.code = 0;
     lp.r_scratch = x->d_rt_scratch;
     lp.r_words_per_cta = x->rt_words_per_cta;
-    const long long slots = 2LL * x->rt_G;
-    const long long want = ((long long)a.n + slots - 1) / slots;
+    // as many CTAs as fill their slots, and a CTA on every SM while there are codewords for it
+    lp.half = rt_half((double)a.n, (double)x->rt_G * x->rt_ctas);
+    const long long slots = (lp.half ? 2LL : 4LL) * x->rt_G;
+    const long long want = std::max(((long long)a.n + slots - 1) / slots, std::min<long long>(a.n, x->sms));
     const int grid = (int)std::min<long long>(want, x->rt_ctas);
     x->rt_kernel<<<grid, x->rt_threads, x->rt_smem, s>>>(lp);
     CUDA_TRY(cudaGetLastError());

@@ -150,19 +150,25 @@ int launch_oms(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s);
 int setup_oms_rt(ldpc_ctx* x);
 int launch_oms_rt(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s);
 // Fill `out` for one code: int8 offset beta8[l] per layer (nullptr: beta8_all on every
-// layer), Max8 as half2 bits, G codeword pairs per CTA.
+// layer), Max8 as half2 bits, G quads of codewords per CTA.
 int make_rt_code(const ldpc_code& c, int max_iter, uint32_t maxv2, const int* beta8, int beta8_all, int G, RtCode* out);
 // Largest row weight the run-time kernels unroll for (0: unsupported).
 int rt_dmax(int max_row_weight);
-// codeword pairs per CTA of the run-time-table kernel for a code of lift Z
+// quads of codewords per CTA of the run-time-table kernel for a code of lift Z
 // and length N: CTAs of at most 128 threads (256 for N > 2048), fewest idle lanes
 int rt_default_G(int z, int n);
 constexpr int kRtMaxThreads = 512;          // __launch_bounds__ of oms_rt_kernel
-constexpr int kRtMaxSmem = 200 * 1024;      // dynamic shared memory the run-time kernels may use
+constexpr int kRtMaxSmem = 206 * 1024;      // dynamic shared memory the run-time kernels may use
 rt_fn rt_kernel_for(int dmax, bool quirk, bool rsmem);
+constexpr int kRtMaxG = 8;                  // quads per CTA: 32 codeword slots, one per lane
 int rt_stride(int n, int G);
-// dynamic shared memory of one CTA: tables, G pairs of posteriors and staging, messages if rsmem
+// dynamic shared memory of one CTA: tables, G quads of posteriors and staging, messages if rsmem
+// (without the staging when that would exceed kRtMaxSmem)
 size_t rt_smem_bytes(int n, int G, int E, int threads, bool rsmem);
+bool rt_nostage(int n, int G, int E);
+// 1: decode n codewords with two per word (2 slots per quad), 0: four; slots =
+// quads that the launch's CTAs hold
+int rt_half(double n, double quads);
 int setup_int(ldpc_ctx* x);
 int launch_int(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s);
 // the decoder of the context's variant

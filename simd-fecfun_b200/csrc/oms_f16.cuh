@@ -63,7 +63,12 @@ __device__ __forceinline__ uint32_t habs2(uint32_t a) { return a & 0x7fff7fffu; 
 __device__ __forceinline__ uint32_t hmin2_xs(uint32_t a, uint32_t b) { uint32_t d; asm("min.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 __device__ __forceinline__ uint32_t hmax2_xs(uint32_t a, uint32_t b) { uint32_t d; asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 
-constexpr uint32_t H2_M128 = 0xd800d800u;   // -128.0 in both lanes
+// a - b clamped to [0, 1]
+__device__ __forceinline__ uint32_t hsub2_sat(uint32_t a, uint32_t b) { uint32_t d; asm("sub.rn.sat.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ uint32_t habs2_f(uint32_t a) { uint32_t d; asm("abs.f16x2 %0, %1;" : "=r"(d) : "r"(a)); return d; }
+
+constexpr uint32_t H2_1408 = 0x65806580u;   // 1408.0 in both lanes
+constexpr uint32_t H2_M128 = 0xd800d800u;   // -128.0
 constexpr uint32_t H2_P127 = 0x57f057f0u;   // +127.0
 constexpr uint32_t H2_ZERO = 0u;
 constexpr uint32_t H2_1024 = 0x64006400u;   // 1024.0

@@ -91,8 +91,9 @@ constexpr int RT_MAX_Z = 511;        // shifts are packed in 9 bits
 // when it starts work on that code.
 struct alignas(16) RtCode {
     int z, n, L, E;
-    int G;                           // codeword pairs per CTA (thread (t, g): check row t, pair g)
-    int stride;                      // posterior words per pair in shared memory
+    int G;                           // quads of codewords per CTA (thread (t, g): check row t, quad g)
+    int stride;                      // posterior words per quad in shared memory
+    int nostage;                     // 1: no LLR staging buffers; slots refilled from global memory
     int kbits, hard_words, num_par, max_iter;
     uint32_t maxv2;                  // half2 bits of Max8
     uint32_t beta2[RT_MAX_L];        // half2 bits of beta8 per layer
@@ -101,7 +102,8 @@ struct alignas(16) RtCode {
     int tab_rows;                    //   (0-based) uses row min(i, tab_rows - 1), in place of beta2 / quirk2
     int16_t rw[RT_MAX_L];
     int16_t ebase[RT_MAX_L];         // first edge of layer l
-    uint32_t edge[RT_MAX_E];         // (column * Z) << 9 | shift
+    int16_t run[RT_MAX_L];           // first layer after l of another weight (or L)
+    SpEdge edge[RT_MAX_E];           // in bytes of a posterior word; a CTA copies E of them
 };
 
 // One batch of codewords of one code (device pointers).
@@ -135,6 +137,8 @@ struct RtLaunch {
     RtJob job0;
     uint32_t* r_scratch;             // check messages in global memory (when not in shared memory)
     long long r_words_per_cta;
+    uint32_t zero;                   // 0 (RtConst)
+    int half;                        // 1: two codewords per word (bytes 0 and 1), 2G slots; 0: four, 4G slots
 };
 
 // ---- fused generation ----
