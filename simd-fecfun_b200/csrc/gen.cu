@@ -45,11 +45,22 @@ size_t gen_tile_shape(const GenTables& t, GenTile* tile) {
     return smem;
 }
 
-int gen_grid(ldpc_ctx* x, long long n, int* smem) {
-    const GenTables& t = x->gent;
-    *smem = gen_warp_words(t.kbits, t.mcol, t.z, t.n) * 4 * 8;
-    const long long want = (n + 7) / 8;
-    return (int)std::max<long long>(1, std::min<long long>(want, (long long)x->sms * 8));
+typedef void (*encode_fn)(const GenTables, const EncodeShape, const uint32_t*, long long, uint8_t*);
+const encode_fn kEncode[] = {encode_kernel<1>, encode_kernel<4>, encode_kernel<8>, encode_kernel<16>};
+
+// Codewords per warp of encode_kernel: as many as their columns' words fill its
+// lanes, within 56 KB per CTA (four CTAs per SM), and no more than give every
+// SM's warps one group (small calls).
+EncodeShape encode_shape(const GenTables& t, long long n, int sms, int* smem) {
+    const int zw = (t.z + 31) / 32;
+    EncodeShape s;
+    const int words = encode_words(t.mcol, zw, t.hard_words);
+    s.stride = words + (((zw - words) % 32) + 32) % 32;
+    s.cws = std::max(1, std::min(32 / zw, 56 * 1024 / (8 * 4 * s.stride)));
+    while (s.cws > 1 && n < (long long)s.cws * 8 * sms) s.cws = (s.cws + 1) / 2;
+    s.inv_z = (uint32_t)(((1ull << 32) + t.z - 1) / t.z);
+    *smem = 8 * 4 * s.cws * s.stride;
+    return s;
 }
 }  // namespace
 
@@ -97,15 +108,14 @@ int setup_gen(ldpc_ctx* x) {
     CUDA_TRY(cudaMemcpy(x->d_masks + t.n, c.filler.data(), t.n, cudaMemcpyHostToDevice));
     t.punct = x->d_masks;
     t.filler = x->d_masks + t.n;
-    int smem = 0;
-    gen_grid(x, 1, &smem);
+    const int smem = gen_warp_words(t.kbits, t.mcol, t.z, t.n) * 4 * 8;
     if (smem > 200 * 1024) return fail(LDPC_ERR_UNSUPPORTED, "generator needs %d B of shared memory", smem);
     GenTile tile;
     const size_t gsmem = gen_tile_shape(t, &tile);
     if (gsmem > 200 * 1024) return fail(LDPC_ERR_UNSUPPORTED, "generator tile needs %zu B of shared memory", gsmem);
     CUDA_TRY(allow_dynamic_smem((const void*)gen_kernel<false>, 200 * 1024));
     CUDA_TRY(allow_dynamic_smem((const void*)gen_kernel<true>, 200 * 1024));
-    CUDA_TRY(allow_dynamic_smem((const void*)encode_kernel, 200 * 1024));
+    for (encode_fn k : kEncode) CUDA_TRY(allow_dynamic_smem((const void*)k, 200 * 1024));
     return LDPC_OK;
 }
 
@@ -214,9 +224,17 @@ int ldpc_encode(ldpc_ctx* x, const uint32_t* data_bits, size_t n, uint8_t* cw_bi
     if (n == 0) return LDPC_OK;
     if (!data_bits || !cw_bits) return fail(LDPC_ERR_INVALID_ARG, "NULL buffer");
     CUDA_TRY(cudaSetDevice(x->device));
+    // the widest store that divides the codeword and whose alignment the output has
+    const ldpc::GenTables& t = x->gent;
+    const unsigned long long al = (unsigned long long)t.n | (unsigned long long)(uintptr_t)cw_bits;
+    const int v = (al & 15) == 0 ? 3 : (al & 7) == 0 ? 2 : (al & 3) == 0 ? 1 : 0;
     int smem = 0;
-    const int grid = ldpc::gen_grid(x, (long long)n, &smem);
-    ldpc::encode_kernel<<<grid, 256, smem, (cudaStream_t)stream>>>(x->gent, data_bits, (long long)n, cw_bits);
+    const ldpc::EncodeShape sh = ldpc::encode_shape(t, (long long)n, x->sms, &smem);
+    int per_sm = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)ldpc::kEncode[v], 256, smem));
+    const long long want = ((long long)n + 8 * sh.cws - 1) / (8 * sh.cws);
+    const int grid = (int)std::min<long long>(want, (long long)x->sms * std::max(per_sm, 1));
+    ldpc::kEncode[v]<<<grid, 256, smem, (cudaStream_t)stream>>>(t, sh, data_bits, (long long)n, cw_bits);
     CUDA_TRY(cudaGetLastError());
     return LDPC_OK;
 }

@@ -552,27 +552,94 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
 }
 
 // QC encoding only: packed data bits -> 0/1 codeword bytes.
-__global__ void __launch_bounds__(256) encode_kernel(const __grid_constant__ GenTables tb, const uint32_t* data_bits,
-                                                     long long n, uint8_t* cw_out) {
+//
+// A warp encodes `cws` codewords at a time, word k of codeword c on lane
+// c * zw + k (zw = ceil(Z/32) words per column), so that every lane works on a
+// parity column: one codeword per warp left 29 of 32 lanes idle at Z = 96, and
+// its output went out one byte per lane.  Columns of one codeword are `stride`
+// words apart from the next one's, stride = zw modulo 32: a warp's lanes fall
+// in distinct banks.  Output: V consecutive bits become V bytes (four at a time
+// by a multiplication that moves bit q to bit 8 q) and one V-byte store.
+// 802.16e 1/2 Z = 96, 65536 codewords (160 MB in and out): 572 -> 76 us.
+struct EncodeShape {
+    int cws, stride;                 // codewords per warp, words per codeword in shared memory
+    uint32_t inv_z;                  // ceil(2^32 / z): c = umulhi(i, inv_z) for i < 2^20
+};
+
+// cols: column c's words at [c * (zw + 1)], a zero word behind them; the data
+// words (hard_words and three zero words) behind the columns.
+__host__ __device__ inline int encode_words(int mcol, int zw, int hard_words) { return mcol * (zw + 1) + hard_words + 3; }
+
+template <int V>
+__global__ void __launch_bounds__(256) encode_kernel(const __grid_constant__ GenTables tb, const EncodeShape sh,
+                                                     const uint32_t* data_bits, long long n, uint8_t* cw_out) {
     extern __shared__ uint32_t sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wpw = gen_warp_words(tb.kbits, tb.mcol, tb.z, tb.n);
-    uint32_t* data = sm + warp * wpw;
-    uint32_t* cols = data + (tb.kbits / 32 + 2);
-    uint32_t* cwbits = cols + tb.mcol * ((tb.z + 31) / 32 + 1);
-    const long long nwarps_total = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long i = (long long)blockIdx.x * (blockDim.x >> 5) + warp; i < n; i += nwarps_total) {
-        const int dw = tb.kbits / 32 + 2;
-        for (int w = lane; w < dw; w += 32) {
-            uint32_t v = w < tb.hard_words ? data_bits[i * tb.hard_words + w] : 0u;
-            const int lo = w * 32;
-            if (lo + 32 > tb.kbits) v &= (lo >= tb.kbits) ? 0u : ((1u << (tb.kbits - lo)) - 1u);
-            data[w] = v;
+    const int z = tb.z, zw = (z + 31) / 32, kc = tb.mcol - tb.mrow, hw = tb.hard_words, nv = tb.n / V;
+    const uint32_t last_mask = (z & 31) ? ((1u << (z & 31)) - 1u) : 0xffffffffu;
+    uint32_t* const mine = sm + warp * sh.cws * sh.stride;
+    const int data_at = tb.mcol * (zw + 1);
+    // spare words: zero for good
+    for (int c = 0; c < sh.cws; ++c) {
+        for (int i = lane; i < tb.mcol; i += 32) mine[c * sh.stride + i * (zw + 1) + zw] = 0u;
+        if (lane < 3) mine[c * sh.stride + data_at + hw + lane] = 0u;
+    }
+    const int pc = lane / zw, pk = lane - pc * zw;   // this lane's codeword and word in the parity pass
+    const long long step = (long long)gridDim.x * (blockDim.x >> 5) * sh.cws;
+    for (long long i0 = ((long long)blockIdx.x * (blockDim.x >> 5) + warp) * sh.cws; i0 < n; i0 += step) {
+        const int m = (int)min((long long)sh.cws, n - i0);
+        __syncwarp();   // the previous codewords are written
+        for (int i = lane; i < m * hw; i += 32) {
+            const int c = i / hw, w = i - c * hw;
+            uint32_t v = data_bits[i0 * hw + i];
+            if (w * 32 + 32 > tb.kbits) v &= (1u << (tb.kbits - w * 32)) - 1u;
+            mine[c * sh.stride + data_at + w] = v;
         }
         __syncwarp();
-        encode_warp(tb, data, cols, cwbits, lane);
-        for (int idx = lane; idx < tb.n; idx += 32) cw_out[i * tb.n + idx] = (cwbits[idx >> 5] >> (idx & 31)) & 1u;
+        for (int i = lane; i < m * kc * zw; i += 32) {
+            const int c = i / (kc * zw), r = i - c * (kc * zw), col = r / zw, k = r - col * zw;
+            uint32_t v = stream_bits32(mine + c * sh.stride + data_at, col * z + 32 * k);
+            if (k == zw - 1) v &= last_mask;
+            mine[c * sh.stride + col * (zw + 1) + k] = v;
+        }
         __syncwarp();
+        uint32_t* const cols = mine + pc * sh.stride;
+        for (int r = 0; r < tb.n_par; ++r) {
+            const int first = tb.par_first[r], cnt = tb.par_cnt[r];
+            if (pc < m) {
+                uint32_t acc = 0;
+#pragma unroll 2
+                for (int q = 0; q < cnt; ++q) {
+                    int p = 32 * pk + gen_term_shift(tb, first + q);
+                    p = p >= z ? p - z : p;
+                    acc ^= col_bits32(cols + gen_term_col(tb, first + q) * (zw + 1), z, p);
+                }
+                if (pk == zw - 1) acc &= last_mask;
+                cols[tb.par_col[r] * (zw + 1) + pk] = acc;
+            }
+            __syncwarp();
+        }
+        uint8_t* const dst = cw_out + i0 * tb.n;
+        for (int j = lane, c = 0, q = lane; j < m * nv; j += 32, q += 32) {
+            while (q >= nv) {
+                q -= nv;
+                ++c;
+            }
+            const int idx = V * q, col = (int)__umulhi((uint32_t)idx, sh.inv_z), p = idx - col * z;
+            const uint32_t* w = mine + c * sh.stride + col * (zw + 1);
+            uint32_t v = stream_bits32(w, p);
+            for (int have = z - p; have < V; have += z) {
+                w += zw + 1;
+                v |= w[0] << have;
+            }
+            uint32_t o[(V + 3) / 4];
+#pragma unroll
+            for (int b = 0; b < (V + 3) / 4; ++b) o[b] = (((v >> (4 * b)) & 15u) * 0x00204081u) & 0x01010101u;
+            if (V == 16) *reinterpret_cast<uint4*>(dst + V * j) = make_uint4(o[0], o[V > 4], o[2 * (V > 8)], o[3 * (V > 8)]);
+            else if (V == 8) *reinterpret_cast<uint2*>(dst + V * j) = make_uint2(o[0], o[V > 4]);
+            else if (V == 4) *reinterpret_cast<uint32_t*>(dst + V * j) = o[0];
+            else dst[j] = (uint8_t)(v & 1u);
+        }
     }
 }
 

@@ -209,3 +209,26 @@ def test_generate_int8_path_matches_float_path(capi, name, n):
     assert np.array_equal(li.cpu().numpy(), np.rint(F).astype(np.int16).astype(np.int8))
     if code.punc_list:
         assert np.all(F[:, :, code.punc_list[0]:code.punc_list[1] + 1] == 0)
+
+
+@pytest.mark.parametrize("offset", [0, 4, 8, 1])
+@pytest.mark.parametrize("name,z,n", [("16e 1/2", 96, 33), ("16e 1/2", 25, 70), ("11n 3/4 z27", None, 1), ("11n 2/3 z81", None, 19),
+                                      ("ITU G.hn 1/2 z14", None, 100), ("11ad 13/16", None, 161),
+                                      ("5GNR_n6400_k1280", None, 11), ("802.3ca", None, 3)])
+def test_encode_shapes(capi, oracle, name, z, n, offset):
+    """Every store width (output offset, N modulo 16), several codewords per
+    warp with a ragged last group, one and more words per column; bytes around
+    the output stay as they are."""
+    import torch
+    from conftest import pack_bits
+    from ldpc_b200 import codes
+    code = codes.make_code(name, z_over=z) if z else codes.code_by_name(name)
+    ctx = capi.Context(capi.Code.from_tables(code), max_iter=2)
+    rng = np.random.default_rng(n)
+    info = rng.integers(0, 2, (n, (code.mcol - code.mrow) * code.z), dtype=np.uint8)
+    data = torch.from_numpy(pack_bits(info).view(np.int32)).cuda()
+    out = torch.full((n * code.n + 32,), 7, dtype=torch.uint8, device="cuda")
+    ctx.encode(data, n, out.data_ptr() + offset)
+    got = out.cpu().numpy()
+    assert np.array_equal(got[offset:offset + n * code.n].reshape(n, code.n), oracle.encode(code, info))
+    assert (got[:offset] == 7).all() and (got[offset + n * code.n:] == 7).all()
