@@ -38,7 +38,7 @@ CompiledCode describe() {
 const CompiledCode kCompiledCode11ad12 = describe<Code11ad12>();
 
 const OmsInst kOmsInst[] = {
-    OMS_SPLIT(Code11ad12, kRw11ad12, 30),
+    OMS_SPLIT(Code11ad12, kRw11ad12, 24),
     OMS_COMPILED(Code11ad12, kRw11ad12),
     OMS_FIXED(Shape11ad12, kRw11ad12),
     OMS_PAD(8, 8), OMS_PAD(12, 8), OMS_PAD(8, 12), OMS_PAD(6, 16), OMS_PAD(4, 16), OMS_PAD(3, 16), OMS_PAD(4, 24),

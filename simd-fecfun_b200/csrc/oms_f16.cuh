@@ -13,13 +13,19 @@
 // (LDPCdecode.cpp:172-197).
 //
 // Why f16x2: every quantity is a small integer (|P| <= 128, |R| <= 127), so
-// IEEE half arithmetic on them is exact, and B200 issues packed half2
-// min/max at full rate and half2 add at half rate, while the byte-SIMD
-// intrinsics (__vsubss4 and friends) are emulated at 8-15 ops/clk/SM.
-// Saturation is an explicit clamp to [-128, 127].  The exclusive minimum uses
-// min1/min2 of |Q| (tracked before the offset; beta, the clamp at 0 and Max8
-// are monotone, so they are applied once per check):
-//   f_j = clamp(min1 - beta8, 0, Max8)  if |Q_j| != min1, else clamp(min2 - ...)
+// IEEE half arithmetic on them is exact, and the byte-SIMD intrinsics
+// (__vsubss4 and friends) are emulated at 8-15 ops/clk/SM.  Minima, logic and
+// permutations issue on the ALU pipe, half-precision multiply-adds on the pipe
+// beside it, 64 lanes per clock each; so what can be a multiply-add is one:
+//   - posteriors are held as u = P + 128 (0..255): each saturation is a
+//     multiply-add that stops at 0 and one minimum (Q = min(max(u - R, 0), 255)
+//     - 128, u' = min(max(Q + (R' + 128), 0), 255)) instead of two of each bound;
+//   - the exclusive minimum uses min1/min2 of |Q| (beta, the clamp at 0 and Max8
+//     are monotone, so they are applied once per check); e = clamp(|Q_j| - min1,
+//     0, 1) is 0 for an edge at the minimum and 1 elsewhere (integers), so
+//     f_j = c2 + e (c1 - c2), c = clamp(min - beta8, 0, Max8).
+// 802.11ad 1/2, 5e6 codewords: 35.6 -> 29.0 ms (ALU operations per edge of a
+// pair 15.8 -> 8.2, ALU pipe 79 % busy in the layers before).
 // For beta8 = 0 the int8 quirk abs8(-128) = -128 makes that edge's m = 0;
 // the BETA0 variant reproduces it.
 //
@@ -63,11 +69,17 @@ __device__ __forceinline__ uint32_t habs2(uint32_t a) { return a & 0x7fff7fffu; 
 __device__ __forceinline__ uint32_t hmin2_xs(uint32_t a, uint32_t b) { uint32_t d; asm("min.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 __device__ __forceinline__ uint32_t hmax2_xs(uint32_t a, uint32_t b) { uint32_t d; asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 
+// max(a * b + c, 0)
+__device__ __forceinline__ uint32_t hfma2_relu(uint32_t a, uint32_t b, uint32_t c) { uint32_t d; asm("fma.rn.relu.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
 // a - b clamped to [0, 1]
 __device__ __forceinline__ uint32_t hsub2_sat(uint32_t a, uint32_t b) { uint32_t d; asm("sub.rn.sat.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 __device__ __forceinline__ uint32_t habs2_f(uint32_t a) { uint32_t d; asm("abs.f16x2 %0, %1;" : "=r"(d) : "r"(a)); return d; }
 
 constexpr uint32_t H2_1408 = 0x65806580u;   // 1408.0 in both lanes
+constexpr uint32_t H2_ONE = 0x3c003c00u;    // 1.0 in both lanes
+constexpr uint32_t H2_MONE = 0xbc00bc00u;   // -1.0
+constexpr uint32_t H2_P128 = 0x58005800u;   // 128.0
+constexpr uint32_t H2_P255 = 0x5bf85bf8u;   // 255.0
 constexpr uint32_t H2_M128 = 0xd800d800u;   // -128.0
 constexpr uint32_t H2_P127 = 0x57f057f0u;   // +127.0
 constexpr uint32_t H2_ZERO = 0u;
@@ -167,8 +179,39 @@ struct PaddedShape {
     static constexpr bool fixed = false;
 };
 
+// Smallest and second smallest of W magnitudes, both lanes at once.  x: signed
+// values; on return mn1's sign bits hold the product of all signs.  Merging
+// two (smallest, second) pairs takes a minimum with sign, a maximum and a
+// three-way minimum, so W values cost about 2.2 W operations in log W steps.
+template <int W>
+struct Min2 {
+    __device__ static __forceinline__ void of(const uint32_t* x, uint32_t& mn1, uint32_t& mn2) {
+        constexpr int H = W / 2 + (W / 2 & 1 && W > 2 ? 1 : 0);   // even left parts: whole pairs
+        uint32_t a1, a2, b1, b2;
+        Min2<H>::of(x, a1, a2);
+        Min2<W - H>::of(x + H, b1, b2);
+        mn1 = hmin2_xs(a1, b1);
+        mn2 = hmin2(hmin2(a2, b2), hmax2(habs2_f(a1), habs2_f(b1)));
+    }
+};
+template <>
+struct Min2<1> {
+    __device__ static __forceinline__ void of(const uint32_t* x, uint32_t& mn1, uint32_t& mn2) {
+        mn1 = x[0];
+        mn2 = H2_1024;
+    }
+};
+template <>
+struct Min2<2> {
+    __device__ static __forceinline__ void of(const uint32_t* x, uint32_t& mn1, uint32_t& mn2) {
+        mn1 = hmin2_xs(x[0], x[1]);
+        mn2 = hmax2(habs2_f(x[0]), habs2_f(x[1]));
+    }
+};
+
 struct OmsConsts {
     uint32_t beta2, maxv2;
+    uint32_t one, mone, top;   // 1, -1, 255 in both lanes, as registers (literals that an instruction cannot encode are moves)
     uint32_t* Rs;        // shared-memory messages of edge slots >= E_REG: Rs[(e - E_REG) * S::RS_STRIDE]
 };
 
@@ -197,48 +240,39 @@ __device__ __forceinline__ void oms_layer(const OmsTables& tb, uint32_t* Ps, uin
                                           const OmsConsts& k, uint32_t& plast) {
     constexpr int D = S::maxd(l);
     constexpr uint32_t SGN = 0x80008000u;
-    uint32_t q[D];
+    uint32_t q[D], a[D];
     int addr[D];
-    uint32_t mn1 = H2_1024, mn2 = H2_1024;
-    uint32_t sx = 0;
+    uint32_t mn1, mn2, sx = 0;
 #pragma unroll
     for (int j = 0; j < D; ++j) {
+        a[j] = H2_1024;
         if (S::has(tb, l, j)) {
             const int e = S::slot(l, j);
             addr[j] = S::addr(tb, e, t, gbase);
-            uint32_t Q = hsub2(Ps[addr[j]], get_r<S>(R, k, e));
-            Q = hmin2(hmax2(Q, H2_M128), H2_P127);
+            q[j] = hadd2(hmin2(hfma2_relu(get_r<S>(R, k, e), k.mone, Ps[addr[j]]), k.top), H2_M128);
             if (BETA0) {
-                const uint32_t a = abs_q<BETA0>(Q);
-                mn2 = hmin2(mn2, hmax2(mn1, a));
-                mn1 = hmin2(mn1, a);
-                sx ^= Q;
+                a[j] = abs_q<BETA0>(q[j]);
+                sx ^= q[j];
             } else {
-                // magnitudes as above; mn1's sign bits accumulate the sign
-                // product (Q is never -0: P and R start at +0 and x - x = +0)
-                mn2 = hmin2_xs(mn2, hmax2_xs(mn1, Q));
-                mn1 = hmin2_xs(mn1, Q);
+                a[j] = q[j];
             }
-            q[j] = Q;
         }
     }
-    if (!BETA0) {
-        sx = mn1;
-        mn1 = habs2(mn1);
-        mn2 = habs2(mn2);
-    }
+    Min2<D>::of(a, mn1, mn2);
+    // mn1's sign bits hold the sign product (Q is never -0: it is a difference that rounds 0 to +0)
+    if (!BETA0) sx = mn1;
+    mn1 = habs2(mn1);
     const uint32_t c1 = hmin2(hmax2(hsub2(mn1, k.beta2), H2_ZERO), k.maxv2);
     const uint32_t c2 = hmin2(hmax2(hsub2(mn2, k.beta2), H2_ZERO), k.maxv2);
-    const uint32_t X = c1 ^ c2;
-    const uint32_t M1 = c1 ^ (sx & SGN);
+    const uint32_t f2 = c2 ^ (sx & SGN), df = hsub2(c1, c2) ^ (sx & SGN);
 #pragma unroll
     for (int j = 0; j < D; ++j) {
         if (S::has(tb, l, j)) {
-            const uint32_t eq = heq2_mask(abs_q<BETA0>(q[j]), mn1);
-            const uint32_t Rn = M1 ^ (q[j] & SGN) ^ (eq & X);
-            const uint32_t Pn = hmin2(hmax2(hadd2(q[j], Rn), H2_M128), H2_P127);
-            Ps[addr[j]] = Pn;
-            if (l == S::L - 1) plast ^= Pn;
+            const uint32_t e = hsub2_sat(BETA0 ? abs_q<BETA0>(q[j]) : habs2_f(q[j]), mn1);
+            const uint32_t Rn = hfma2(e, df, f2) ^ (q[j] & SGN);
+            const uint32_t un = hmin2(hfma2_relu(q[j], k.one, hadd2(Rn, H2_P128)), k.top);
+            Ps[addr[j]] = un;
+            if (l == S::L - 1) plast ^= hadd2(un, H2_M128);
             set_r<S>(R, k, S::slot(l, j), Rn);
         }
     }
@@ -267,7 +301,7 @@ __device__ __forceinline__ uint32_t oms_row_parity(const OmsTables& tb, const ui
     uint32_t x = 0;
 #pragma unroll
     for (int j = 0; j < S::maxd(l); ++j) {
-        if (S::has(tb, l, j)) x ^= Ps[S::addr(tb, S::slot(l, j), t, gbase)];
+        if (S::has(tb, l, j)) x ^= hadd2(Ps[S::addr(tb, S::slot(l, j), t, gbase)], H2_M128);
     }
     return x;
 }
@@ -307,7 +341,8 @@ __device__ __forceinline__ void oms_syndrome_loop(const OmsTables& tb, const uin
         const int d = tb.rw[l];
         const int base = S::fixed ? e0 : l * tb.D;
         uint32_t x = 0;
-        for (int j = 0; j < d; ++j) x ^= Ps[gbase + tb.colz[base + j] + wrap_add(t, tb.shift[base + j], tb.z)];
+        for (int j = 0; j < d; ++j)
+            x ^= hadd2(Ps[gbase + tb.colz[base + j] + wrap_add(t, tb.shift[base + j], tb.z)], H2_M128);
         e0 += d;
         x &= 0x80008000u;
         if (x & ~seen) {
@@ -380,7 +415,7 @@ __global__ void __launch_bounds__(MAXT, MINB) oms_f16_kernel(const __grid_consta
     const long long lo = job.ncw * blockIdx.x / gridDim.x, hi = job.ncw * (blockIdx.x + 1) / gridDim.x;
 
     for (int i = tid; i < OMS_MAX_BUCKETS * 4; i += blockDim.x) (&s_cnt[0][0])[i] = 0;
-    for (int i = tid; i < G * stride; i += blockDim.x) Ps[i] = 0;
+    for (int i = tid; i < G * stride; i += blockDim.x) Ps[i] = H2_P128;   // P = 0
     if (tid < 32) {
         const long long c0 = lo + tid, c1 = lo + nslots + tid;
         const bool ok = tid < nslots;
@@ -408,7 +443,7 @@ __global__ void __launch_bounds__(MAXT, MINB) oms_f16_kernel(const __grid_consta
         if (s_cur[k] >= 0) {
             __half* dst = reinterpret_cast<__half*>(Ps + (k >> 1) * stride) + (k & 1);
             const int8_t* st = stage_base + k * nstage;
-            for (int i = lane; i < n; i += 32) dst[2 * i] = __int2half_rn((int)st[i]);
+            for (int i = lane; i < n; i += 32) dst[2 * i] = __int2half_rn((int)st[i] + 128);
         }
         __syncwarp();
         if (s_next[k] >= 0) prefetch_llr(stage_base + k * nstage, job.llr, s_next[k], n, lane);
@@ -423,6 +458,9 @@ __global__ void __launch_bounds__(MAXT, MINB) oms_f16_kernel(const __grid_consta
     OmsConsts kc;
     kc.beta2 = job.beta2;
     kc.maxv2 = job.maxv2;
+    kc.one = H2_ONE ^ job.zero;
+    kc.mone = H2_MONE ^ job.zero;
+    kc.top = H2_P255 ^ job.zero;
     // shared-memory messages after the LLR staging area
     kc.Rs = reinterpret_cast<uint32_t*>(stage_base + 2 * G * nstage) + tid;
     for (int e = S::E_REG; e < S::E; ++e) kc.Rs[(e - S::E_REG) * S::RS_STRIDE] = 0u;
@@ -483,12 +521,12 @@ __global__ void __launch_bounds__(MAXT, MINB) oms_f16_kernel(const __grid_consta
             // hard decisions of the data columns, 32 per ballot; error counts
             const uint32_t* ref = job.ref_bits ? job.ref_bits + (cw % job.ref_period) * tb.hard_words : nullptr;
             unsigned errw, errslots;
-            warp_hard_decisions<false>([&](int i) { return __hlt(pk[2 * i], __float2half(0.0f)); }, tb.kbits, tb.hard_words, z,
+            warp_hard_decisions<false>([&](int i) { return __hlt(pk[2 * i], __float2half(128.0f)); }, tb.kbits, tb.hard_words, z,
                                 job.num_par, job.hard_out ? job.hard_out + cw * tb.hard_words : nullptr, ref, lane, errw,
                                 errslots);
             if (job.post_out) {
                 int8_t* dst = job.post_out + cw * (long long)n;
-                for (int i = lane; i < n; i += 32) dst[i] = (int8_t)__half2int_rn(pk[2 * i]);
+                for (int i = lane; i < n; i += 32) dst[i] = (int8_t)(__half2int_rn(pk[2 * i]) - 128);
             }
             if (lane == 0 && job.iters_out) job.iters_out[cw] = (uint8_t)it;
             if (job.counters && lane == 0) {
@@ -506,7 +544,7 @@ __global__ void __launch_bounds__(MAXT, MINB) oms_f16_kernel(const __grid_consta
             const long long nxt = s_next[k];
             if (nxt >= 0) {
                 const int8_t* st = stage_base + k * nstage;
-                for (int i = lane; i < n; i += 32) pk[2 * i] = __int2half_rn((int)st[i]);
+                for (int i = lane; i < n; i += 32) pk[2 * i] = __int2half_rn((int)st[i] + 128);
                 __syncwarp();
                 unsigned long long c = 0;
                 if (lane == 0) c = atomicAdd(&s_head, 1ull);

@@ -81,36 +81,6 @@ __device__ __forceinline__ uint32_t* rt_at(SpEdge e, char* Pg, uint32_t tb, uint
     return reinterpret_cast<uint32_t*>(Pg + (e.col + min(w, w + zb)));
 }
 
-// Smallest and second smallest of W magnitudes, both lanes at once.  x: signed
-// values; on return mn1's sign bits hold the product of all signs.  Merging
-// two (smallest, second) pairs takes a minimum with sign, a maximum and a
-// three-way minimum, so W values cost about 2.2 W operations in log W steps.
-template <int W>
-struct Min2 {
-    __device__ static __forceinline__ void of(const uint32_t* x, uint32_t& mn1, uint32_t& mn2) {
-        constexpr int H = W / 2 + (W / 2 & 1 && W > 2 ? 1 : 0);   // even left parts: whole pairs
-        uint32_t a1, a2, b1, b2;
-        Min2<H>::of(x, a1, a2);
-        Min2<W - H>::of(x + H, b1, b2);
-        mn1 = hmin2_xs(a1, b1);
-        mn2 = hmin2(hmin2(a2, b2), hmax2(habs2_f(a1), habs2_f(b1)));
-    }
-};
-template <>
-struct Min2<1> {
-    __device__ static __forceinline__ void of(const uint32_t* x, uint32_t& mn1, uint32_t& mn2) {
-        mn1 = x[0];
-        mn2 = H2_1024;
-    }
-};
-template <>
-struct Min2<2> {
-    __device__ static __forceinline__ void of(const uint32_t* x, uint32_t& mn1, uint32_t& mn2) {
-        mn1 = hmin2_xs(x[0], x[1]);
-        mn2 = hmax2(habs2_f(x[0]), habs2_f(x[1]));
-    }
-};
-
 // Constants of a row's update, kept in registers: as literals each use of one
 // that its instruction cannot encode is a move of its own (5 of 45 operations
 // per quad's edge).
