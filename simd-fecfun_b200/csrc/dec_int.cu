@@ -104,7 +104,7 @@ int launch_int(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     job.beta = x->ibeta;
     job.maxv = x->imaxv;
     job.r_scratch = (int32_t*)x->d_int_scratch;
-    const long long want = ((long long)a.n + x->spt.G - 1) / x->spt.G;
+    const long long want = spread_ctas(a.n, x->spt.G, x->sms);
     const int grid = (int)std::min<long long>(want, x->int_ctas);
     ((int_fn)x->int_kernel)<<<grid, x->int_threads, x->int_smem, s>>>(x->spt, job);
     CUDA_TRY(cudaGetLastError());

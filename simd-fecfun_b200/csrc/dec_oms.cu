@@ -189,8 +189,7 @@ int launch_oms(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     job.queue = x->d_queue + a.queue;
     job.status = x->d_status;
     job.synd_loop = x->oms_synd_loop;
-    const long long slots = 2LL * x->omst.G;
-    const long long want = ((long long)a.n + slots - 1) / slots;
+    const long long want = spread_ctas(a.n, 2LL * x->omst.G, x->sms);
     const int grid = (int)std::min<long long>(want, x->oms_ctas);
     oms_fn k = x->beta0 ? x->oms_launch->k_beta0 : x->oms_launch->k_beta;
     k<<<grid, x->oms_threads, x->oms_smem, s>>>(x->omst, job);

@@ -190,10 +190,8 @@ int launch_oms_rt(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     j.code = 0;
     lp.r_scratch = x->d_rt_scratch;
     lp.r_words_per_cta = x->rt_words_per_cta;
-    // as many CTAs as fill their slots, and a CTA on every SM while there are codewords for it
     lp.half = rt_half((double)a.n, (double)x->rt_G * x->rt_ctas);
-    const long long slots = (lp.half ? 2LL : 4LL) * x->rt_G;
-    const long long want = std::max(((long long)a.n + slots - 1) / slots, std::min<long long>(a.n, x->sms));
+    const long long want = spread_ctas(a.n, (lp.half ? 2LL : 4LL) * x->rt_G, x->sms);
     const int grid = (int)std::min<long long>(want, x->rt_ctas);
     x->rt_kernel<<<grid, x->rt_threads, x->rt_smem, s>>>(lp);
     CUDA_TRY(cudaGetLastError());

@@ -162,7 +162,7 @@ SpJobT<T> sp_job(const ldpc_ctx* x, const DecodeArgs& a, T maxv) {
 int launch_sp(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     if (!x->sp_kernel && !x->sp64_kernel) return fail(LDPC_ERR_INVALID_ARG, "context was not created for a float decoder");
     if (a.n == 0) return LDPC_OK;
-    const long long want = ((long long)a.n + x->spt.G - 1) / x->spt.G;
+    const long long want = spread_ctas(a.n, x->spt.G, x->sms);
     const int grid = (int)std::min<long long>(want, x->sp_ctas);
     if (x->sp64_kernel)
         x->sp64_kernel<<<grid, x->sp_threads, x->sp_smem, s>>>(x->spt, sp_job<double>(x, a, x->maxd));

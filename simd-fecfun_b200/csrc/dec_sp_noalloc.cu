@@ -177,7 +177,7 @@ extern "C" int ldpc_decode_f32_noalloc(const ldpc_code* code, const ldpc_cfg* cf
     // decode_row's Max_row_simd (decode_functions.cpp:27-32) for a float build
     job.maxv = cfg->max_row_metric < 1e-6 ? (float)(1.0 - (double)cfg->max_row_metric) : cfg->max_row_metric;
     job.r_scratch = ds->scratch;
-    const long long want = ((long long)n + G - 1) / G;
+    const long long want = ldpc::spread_ctas(n, G, ds->sms);
     const long long cap = std::min<long long>((long long)per_sm * ds->sms, (long long)(kScratchBytes / per_cta));
     const int grid = (int)std::min(want, cap);
     k<<<grid, threads, smem, (cudaStream_t)stream>>>(t, job);

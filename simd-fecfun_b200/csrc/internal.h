@@ -54,6 +54,15 @@ struct OmsInst {
     OmsLaunch launch[4];
 };
 
+// CTAs that n codewords go to, `slots` per CTA: no more than fill their slots,
+// but a CTA on every SM while there are codewords for it (a few codewords then
+// run side by side on as many SMs, each with short slot phases, not one after
+// the other's).
+inline long long spread_ctas(size_t n, long long slots, int sms) {
+    const long long m = (long long)n, want = (m + slots - 1) / slots;
+    return want > sms ? want : m < sms ? m : sms;
+}
+
 // Arguments of one decode launch (device pointers).
 struct DecodeArgs {
     const void* llr = nullptr;
@@ -141,6 +150,9 @@ struct ldpc_ctx {
     // host-buffer pipeline: per stream, device buffers for one chunk (grow-only)
     void* d_pipe[2][4] = {{nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}};
     size_t pipe_bytes[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    // host-buffer calls of up to kSmallHost bytes in and out: pinned copy of both
+    static constexpr size_t kSmallHost = 256 * 1024;
+    uint8_t* h_small = nullptr;
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
 };
 
