@@ -58,12 +58,13 @@ int setup_int(ldpc_ctx* x) {
     const size_t r_smem = (size_t)(t.E | 1) * threads * 4;   // shared: odd per-thread stride
     const size_t r_glob = (size_t)t.E * threads * 4;          // global scratch: edge-major
     const bool rsmem = base + r_smem <= 160 * 1024;
-    const size_t smem = base + (rsmem ? r_smem : 0);
-    if (smem > (size_t)kSpMaxSmem) return fail(LDPC_ERR_UNSUPPORTED, "int%d decoder: %zu B of shared memory", bits, smem);
+    const size_t payload = base + (rsmem ? r_smem : 0), smem = payload + sp_edge_bytes(t.E);
+    if (payload > (size_t)kSpMaxSmem)
+        return fail(LDPC_ERR_UNSUPPORTED, "int%d decoder: %zu B of shared memory", bits, payload);
     const IntVariant* v = nullptr;
     for (const IntVariant& k : kInt)
         if (k.bits == bits && k.dmax == dmax && k.rsmem == rsmem) v = &k;
-    CUDA_TRY(allow_dynamic_smem((const void*)v->k, kSpMaxSmem));
+    CUDA_TRY(allow_dynamic_smem((const void*)v->k, kSpMaxSmem + kSpEdgeSmem));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)v->k, threads, smem));
     if (per_sm < 1) return fail(LDPC_ERR_UNSUPPORTED, "int%d decoder: launch does not fit an SM", bits);

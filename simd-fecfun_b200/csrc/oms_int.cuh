@@ -10,6 +10,8 @@
 // Values are held as sign-extended int32 in shared memory, one codeword per
 // group of Z threads (thread (t, g) = check row t of every layer), with the
 // run-time tables, slot refill and fused counting of the float decoder.
+// Straight-line rows, the magnitude kept from the first pass: 802.11ad 1/2
+// int16, 100005 codewords 2.89 -> 1.95 ms.
 #pragma once
 #include <stdint.h>
 
@@ -60,38 +62,38 @@ __device__ __forceinline__ int32_t int_abs(int32_t q) {
     return q < 0 ? int_wrap<W>((int32_t)(0u - (uint32_t)q)) : q;
 }
 
-template <int W, int DMAX>
-__device__ __forceinline__ void int_layer(const SpTables& tb, int l, char* Pg, int32_t* Rt, int rstride, uint32_t tb_,
-                                          uint32_t zb, int beta, int maxv) {
-    const int d = tb.rw[l], eb = tb.ebase[l];
-    int32_t q[DMAX];
-    int32_t* p[DMAX];
+// One row's update (LO <= d <= WD edges from table entry ed, messages R[j *
+// rstride]), straight-line as the float decoders' sp_row.
+template <int W, int LO, int WD>
+__device__ __forceinline__ void int_row(const SpEdge* ed, int d, char* Pg, int32_t* R, int rstride, uint32_t tb_, uint32_t zb,
+                                        int beta, int maxv) {
+    int32_t* p[WD];
+    int32_t q[WD], m[WD];
     int32_t mn1 = 0x7fffffff, mn2 = 0x7fffffff;
     uint32_t rx = 0;
 #pragma unroll
-    for (int j = 0; j < DMAX; ++j) {
-        if (j < d) {
-            const int e = eb + j;
-            p[j] = sp_at<int32_t>(tb.edge[e], Pg, tb_, zb);
-            const int32_t Q = int_sat<W>(*p[j], Rt[e * rstride], true);
-            int32_t m = int_wrap<W>(int_abs<W>(Q) - beta);
-            m = m > 0 ? m : 0;
-            mn2 = min(mn2, max(mn1, m));
-            mn1 = min(mn1, m);
-            rx ^= (uint32_t)Q;
-            q[j] = Q;
+    for (int j = 0; j < WD; ++j) {
+        const int e = j < LO ? j : min(j, d - 1);
+        p[j] = sp_at<int32_t>(ed[e], Pg, tb_, zb);
+        q[j] = int_sat<W>(*p[j], R[e * rstride], true);
+    }
+#pragma unroll
+    for (int j = 0; j < WD; ++j) {
+        m[j] = max(int_wrap<W>(int_abs<W>(q[j]) - beta), 0);
+        if (j < LO || j < d) {
+            mn2 = min(mn2, max(mn1, m[j]));
+            mn1 = min(mn1, m[j]);
+            rx ^= (uint32_t)q[j];
         }
     }
     const int32_t f1 = min(maxv, mn1), f2 = min(maxv, mn2);
 #pragma unroll
-    for (int j = 0; j < DMAX; ++j) {
-        if (j < d) {
-            int32_t m = int_wrap<W>(int_abs<W>(q[j]) - beta);
-            m = m > 0 ? m : 0;
-            const int32_t f = m == mn1 ? f2 : f1;
-            const int32_t rn = ((rx ^ (uint32_t)q[j]) & 0x80000000u) ? -f : f;
+    for (int j = 0; j < WD; ++j) {
+        const int32_t f = m[j] == mn1 ? f2 : f1;
+        const int32_t rn = ((rx ^ (uint32_t)q[j]) & 0x80000000u) ? -f : f;
+        if (j < LO || j < d) {
             *p[j] = int_sat<W>(q[j], rn, false);
-            Rt[(eb + j) * rstride] = rn;
+            R[j * rstride] = rn;
         }
     }
 }
@@ -133,8 +135,9 @@ __global__ void __launch_bounds__(512) oms_int_kernel(const __grid_constant__ Sp
     const int t = tid / G, g = tid - (tid / G) * G;
     const bool active = t < z;
     const int gbase = g * stride;
-    int32_t* Ps = sm_i;
-    TL* stage = reinterpret_cast<TL*>(sm_i + ((G * stride + 3) & ~3));        // [G][nstage], 16-byte aligned
+    const SpEdge* edges = sp_load_edges(tb, sm_i);
+    int32_t* Ps = sm_i + sp_edge_bytes(tb.E) / 4;
+    TL* stage = reinterpret_cast<TL*>(Ps + ((G * stride + 3) & ~3));        // [G][nstage], 16-byte aligned
     const int nstage = ((n * (int)sizeof(TL) + 15) & ~15) / (int)sizeof(TL);
     int32_t* Rbase = RSMEM ? reinterpret_cast<int32_t*>(stage + G * nstage)
                            : job.r_scratch + (long long)blockIdx.x * tb.E * nthr;
@@ -177,7 +180,13 @@ __global__ void __launch_bounds__(512) oms_int_kernel(const __grid_constant__ Sp
 
     for (int par = 0;; par ^= 1) {
         for (int l = 0; l < tb.L; ++l) {
-            if (active) int_layer<W, DMAX>(tb, l, Pg, Rt, rstride, tb_, zb, job.beta, job.maxv);
+            if (active) {
+                const int d = tb.rw[l], eb = tb.ebase[l];
+                sp_widths<DMAX>(d, [&](auto lo_, auto w_) {
+                    int_row<W, decltype(lo_)::value, decltype(w_)::value>(edges + eb, d, Pg, Rt + eb * rstride, rstride, tb_, zb,
+                                                                         job.beta, job.maxv);
+                });
+            }
             __syncthreads();
         }
         if (tid == 0) {
@@ -191,10 +200,8 @@ __global__ void __launch_bounds__(512) oms_int_kernel(const __grid_constant__ Sp
                 if (*reinterpret_cast<volatile uint32_t*>(&s_synd[par]) & (1u << g)) break;
                 const int d = tb.rw[l], eb = tb.ebase[l];
                 uint32_t xr = 0;
-                for (int j = 0; j < d; ++j) {
-                    const int e = eb + j;
-                    xr ^= (uint32_t)*sp_at<int32_t>(tb.edge[e], Pg, tb_, zb);
-                }
+#pragma unroll 4
+                for (int j = 0; j < d; ++j) xr ^= (uint32_t)*sp_at<int32_t>(edges[eb + j], Pg, tb_, zb);
                 if (xr & 0x80000000u) {
                     atomicOr(&s_synd[par], 1u << g);
                     break;
