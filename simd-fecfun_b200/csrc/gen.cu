@@ -45,6 +45,8 @@ size_t gen_tile_shape(const GenTables& t, GenTile* tile) {
     return smem;
 }
 
+typedef void (*gen_fn)(const GenTables, const GenJob, const GenTile);
+const gen_fn kGen[2][2] = {{gen_kernel<false, false>, gen_kernel<false, true>}, {gen_kernel<true, false>, gen_kernel<true, true>}};   // [punctured or filler bits][int8 path]
 typedef void (*encode_fn)(const GenTables, const EncodeShape, const uint32_t*, long long, uint8_t*);
 const encode_fn kEncode[] = {encode_kernel<1>, encode_kernel<4>, encode_kernel<8>, encode_kernel<16>};
 
@@ -113,8 +115,8 @@ int setup_gen(ldpc_ctx* x) {
     GenTile tile;
     const size_t gsmem = gen_tile_shape(t, &tile);
     if (gsmem > 200 * 1024) return fail(LDPC_ERR_UNSUPPORTED, "generator tile needs %zu B of shared memory", gsmem);
-    CUDA_TRY(allow_dynamic_smem((const void*)gen_kernel<false>, 200 * 1024));
-    CUDA_TRY(allow_dynamic_smem((const void*)gen_kernel<true>, 200 * 1024));
+    for (const auto& row : kGen)
+        for (gen_fn k : row) CUDA_TRY(allow_dynamic_smem((const void*)k, 200 * 1024));
     for (encode_fn k : kEncode) CUDA_TRY(allow_dynamic_smem((const void*)k, 200 * 1024));
     return LDPC_OK;
 }
@@ -191,14 +193,19 @@ int launch_gen(ldpc_ctx* x, uint64_t seed, uint64_t cw_offset, const float* snr_
         else
             while (tile.T > 1 && (long long)tile.T * nb > cap) tile.T /= 2;
     }
+    // Few codewords: smaller tiles, so that every SM has some (802.16e Z = 96, 512 codewords of
+    // float LLRs in tiles of 32 went to 16 CTAs: 359 us, 106 us in tiles
+    // of 8; 802.11ad, 1000 codewords at 5 points: 85 -> 58 us).  The thread encoder keeps a
+    // warp's worth.
+    const int least = tile.thread_enc ? 32 : GEN_THREADS / 32;
+    while (tile.T > least && (long long)n_per_snr < 2LL * tile.T * x->sms) tile.T /= 2;
     const bool pf = x->gent.any_punct || x->gent.any_filler;
-    const void* kfn = pf ? (const void*)gen_kernel<true> : (const void*)gen_kernel<false>;
+    const gen_fn k = kGen[pf][tile.fast];
     int per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, GEN_THREADS, smem));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, GEN_THREADS, smem));
     const long long tiles = ((long long)n_per_snr + tile.T - 1) / tile.T;
     const int grid = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)x->sms * std::max(per_sm, 1)));
-    if (pf) gen_kernel<true><<<grid, GEN_THREADS, smem, s>>>(x->gent, job, tile);
-    else gen_kernel<false><<<grid, GEN_THREADS, smem, s>>>(x->gent, job, tile);
+    k<<<grid, GEN_THREADS, smem, s>>>(x->gent, job, tile);
     CUDA_TRY(cudaGetLastError());
     return LDPC_OK;
 }

@@ -404,8 +404,9 @@ __device__ __forceinline__ void gen_items_fast(const GenTables& tb, const GenJob
 }
 
 // PF: the code has punctured or filler bits (their masks are applied in the
-// int8 path only then).
-template <bool PF>
+// int8 path only then).  FAST: the int8 path (tile.fast); a kernel of its own,
+// since each path's registers would spill the other's.
+template <bool PF, bool FAST>
 __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_constant__ GenTables tb,
                                                           const __grid_constant__ GenJob job, const GenTile tile) {
     extern __shared__ __align__(16) uint32_t sm[];
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
         }
         __syncthreads();
         // ---- phase B: noise and LLRs, item f = codeword c, block b of 4 bits ----
-        if (tile.fast) {
+        if (FAST) {
             switch (tile.qshift) {
             case 2: gen_items_fast<16, PF>(tb, job, bits, T, i0, tc, tid, tile.clamp16, unc_f); break;
             case 1: gen_items_fast<8, PF>(tb, job, bits, T, i0, tc, tid, tile.clamp16, unc_f); break;
@@ -473,6 +474,10 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
             // (c, b) of item f advanced by GEN_THREADS items per step, without a division per item
             int c = tid / nb, b = tid - (tid / nb) * nb;
             const int step_c = GEN_THREADS / nb, step_b = GEN_THREADS - step_c * nb;
+            // 16-byte stores of wider integers and doubles: whole blocks, aligned output
+            const unsigned long long at = reinterpret_cast<unsigned long long>(job.llr_i16) | reinterpret_cast<unsigned long long>(job.llr_i32) |
+                                          reinterpret_cast<unsigned long long>(job.llr_f64);
+            const bool wide = ((tb.n & 3) | (int)(at & 15)) == 0;
             for (int f = tid; f < tc * nb; f += GEN_THREADS, c += step_c, b += step_b) {
                 if (b >= nb) {
                     b -= nb;
@@ -486,24 +491,36 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
                 const float nz[4] = {g0.x, g0.y, g1.x, g1.y};
                 const int idx0 = 4 * b;
                 const uint32_t bits4 = (bits[(idx0 >> 5) * T + c] >> (idx0 & 31)) & 0xfu;
+                // masks once per block, not per SNR point
+                int pn[4] = {0, 0, 0, 0}, fl[4] = {0, 0, 0, 0};
+                const int m = min(4, tb.n - idx0);
+                if (PF) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (tb.any_punct && q < m) pn[q] = tb.punct[idx0 + q];
+                        if (tb.any_filler && q < m) fl[q] = tb.filler[idx0 + q];
+                    }
+                }
+                const unsigned peers = __activemask();
                 for (int s = 0; s < job.n_snr; ++s) {
                     float l[4];
-                    uint32_t packed = 0;
                     unsigned e = 0;
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const int idx = idx0 + q;
-                        if (idx < tb.n) {
-                            const int pn = tb.any_punct ? tb.punct[idx] : 0;
-                            const int fl = tb.any_filler ? tb.filler[idx] : 0;
-                            e += llr_element((bits4 >> q) & 1u, nz[q], job.sigma[s], job.sigma_factor[s], job.max_abs, pn,
-                                             fl, &l[q]);
-                            packed |= (uint32_t)(uint8_t)llr_to_i8(l[q]) << (8 * q);
-                        }
+                        const unsigned eq = llr_element((bits4 >> q) & 1u, nz[q], job.sigma[s], job.sigma_factor[s],
+                                                        job.max_abs, pn[q], fl[q], &l[q]);
+                        e += q < m ? eq : 0u;
                     }
-                    if (e && job.uncoded) atomicAdd(&s_unc[s], (unsigned long long)e);
+                    if (job.uncoded) {
+                        // one add per warp and SNR point
+                        const unsigned sum = __reduce_add_sync(peers, e);
+                        if (lane == __ffs(peers) - 1 && sum) atomicAdd(&s_unc[s], (unsigned long long)sum);
+                    }
                     const long long row = (long long)s * job.n_per_snr + i;
                     if (job.llr_i8) {
+                        uint32_t packed = 0;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) packed |= (uint32_t)(uint8_t)llr_to_i8(l[q]) << (8 * q);
                         int8_t* dst = job.llr_i8 + row * tb.n + idx0;
                         if ((tb.n & 3) == 0) {
                             *reinterpret_cast<uint32_t*>(dst) = packed;
@@ -511,15 +528,35 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
                             for (int q = 0; q < 4 && idx0 + q < tb.n; ++q) dst[q] = (int8_t)(packed >> (8 * q));
                         }
                     }
-                    if (job.llr_i16 || job.llr_i32) {
-                        for (int q = 0; q < 4 && idx0 + q < tb.n; ++q) {
-                            const int v = __float2int_rn(l[q]);           // roundi (nearest-even)
-                            if (job.llr_i16) job.llr_i16[row * tb.n + idx0 + q] = (int16_t)v;   // compress: wrap to 16 bits
-                            if (job.llr_i32) job.llr_i32[row * tb.n + idx0 + q] = v;
+                    // whole blocks of aligned rows in one or two stores
+                    if (job.llr_i16) {
+                        int v[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) v[q] = __float2int_rn(l[q]);   // roundi (nearest-even), then wrap to 16 bits
+                        int16_t* dst = job.llr_i16 + row * tb.n + idx0;
+                        if (wide) {
+                            *reinterpret_cast<uint2*>(dst) = make_uint2(__byte_perm(v[0], v[1], 0x5410), __byte_perm(v[2], v[3], 0x5410));
+                        } else {
+                            for (int q = 0; q < m; ++q) dst[q] = (int16_t)v[q];
+                        }
+                    }
+                    if (job.llr_i32) {
+                        int32_t* dst = job.llr_i32 + row * tb.n + idx0;
+                        if (wide) {
+                            *reinterpret_cast<int4*>(dst) = make_int4(__float2int_rn(l[0]), __float2int_rn(l[1]),
+                                                                      __float2int_rn(l[2]), __float2int_rn(l[3]));
+                        } else {
+                            for (int q = 0; q < m; ++q) dst[q] = __float2int_rn(l[q]);
                         }
                     }
                     if (job.llr_f64) {
-                        for (int q = 0; q < 4 && idx0 + q < tb.n; ++q) job.llr_f64[row * tb.n + idx0 + q] = (double)l[q];
+                        double* dst = job.llr_f64 + row * tb.n + idx0;
+                        if (wide) {
+                            *reinterpret_cast<double2*>(dst) = make_double2((double)l[0], (double)l[1]);
+                            *reinterpret_cast<double2*>(dst + 2) = make_double2((double)l[2], (double)l[3]);
+                        } else {
+                            for (int q = 0; q < m; ++q) dst[q] = (double)l[q];
+                        }
                     }
                     if (job.llr_f32) {
                         float* dst = job.llr_f32 + row * tb.n + idx0;
@@ -532,7 +569,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
                 }
             }
         }
-        if (tile.fast && job.uncoded) {
+        if (FAST && job.uncoded) {
             // fold the byte counters of this tile (each byte < 256)
 #pragma unroll
             for (int s = 0; s < GEN_FAST_SNR; ++s) {

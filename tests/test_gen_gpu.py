@@ -232,3 +232,31 @@ def test_encode_shapes(capi, oracle, name, z, n, offset):
     got = out.cpu().numpy()
     assert np.array_equal(got[offset:offset + n * code.n].reshape(n, code.n), oracle.encode(code, info))
     assert (got[:offset] == 7).all() and (got[offset + n * code.n:] == 7).all()
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("name,n", [("11ad 1/2", 3), ("11ad 1/2", 700), ("16e 1/2", 130), ("5GNR_n3136_k576", 40)])
+@pytest.mark.parametrize("bits", [16, 32, 64])
+def test_wide_outputs_are_the_float_llrs(capi, bits, name, n, offset):
+    """int16, int32 and double LLRs against the float ones of the same seed
+    (rounded half-even, or widened), stored whole or, at an unaligned base,
+    element by element; the uncoded error counts agree."""
+    import torch
+    from ldpc_b200 import codes
+    code = capi.Code.from_tables(codes.code_by_name(name))
+    kw = dict(max_row_metric=31.0, beta=1.0, llr_scale=8.0, max_abs_llr=500.0)
+    variant, dt = {16: (capi.LDPC_INT16_OMS, torch.int16), 32: (capi.LDPC_INT32_OMS, torch.int32),
+                   64: (capi.LDPC_F64_OMS, torch.float64)}[bits]
+    snrs, N = [-1.0, 0.0, 2.0], code.info.n
+    f = torch.empty((3, n, N), dtype=torch.float32, device="cuda")
+    uf, uw = torch.zeros(3, dtype=torch.int64, device="cuda"), torch.zeros(3, dtype=torch.int64, device="cuda")
+    capi.Context(code, variant=capi.LDPC_F32_OMS, **kw).generate(9, 5, snrs, n, llr_f32=f, uncoded=uf)
+    w = torch.full((3 * n * N + 8,), 77, dtype=dt, device="cuda")
+    capi.Context(code, variant=variant, **kw).generate(9, 5, snrs, n, uncoded=uw,
+                                                                  llr_int=w.data_ptr() + offset * w.element_size())
+    torch.cuda.synchronize()
+    got = w[offset:offset + f.numel()].view(f.shape)
+    want = f.double() if bits == 64 else torch.round(f).to(dt)
+    assert torch.equal(got, want)
+    assert (w[:offset] == 77).all() and (w[offset + f.numel():] == 77).all()
+    assert torch.equal(uf, uw)
