@@ -180,15 +180,14 @@ int float_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int thread
             if (used[c]) m = std::max(m, base[c] + (rs ? (size_t)((int)b->codes[c].row_cols.size() | 1) * threads * 4 : 0));
         return m;
     };
-    if (rsmem && prod) {
-        // as for a single code: sum-product keeps shared-memory messages
-        // unless global (L2) messages give at least 1.5 times the CTAs per SM
+    if (rsmem) {
+        // as for a single code
         int per_s = 0, per_g = 0;
         CUDA_TRY(ldpc::allow_dynamic_smem((const void*)find(true), kSpBatchSmem));
         CUDA_TRY(ldpc::allow_dynamic_smem((const void*)find(false), kSpBatchSmem));
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_s, (const void*)find(true), threads, smem_of(true)));
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_g, (const void*)find(false), threads, smem_of(false)));
-        rsmem = 2 * per_g < 3 * per_s;
+        rsmem = ldpc::messages_in_smem(prod, per_s, per_g);
     }
     const size_t smem = smem_of(rsmem);
     spb_fn k = find(rsmem);

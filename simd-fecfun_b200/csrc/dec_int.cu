@@ -57,13 +57,30 @@ int setup_int(ldpc_ctx* x) {
     const size_t base = ((((size_t)G * t.stride + 3) & ~(size_t)3) * 4) + (size_t)G * nstage_bytes;
     const size_t r_smem = (size_t)(t.E | 1) * threads * 4;   // shared: odd per-thread stride
     const size_t r_glob = (size_t)t.E * threads * 4;          // global scratch: edge-major
-    const bool rsmem = base + r_smem <= 160 * 1024;
-    const size_t payload = base + (rsmem ? r_smem : 0), smem = payload + sp_edge_bytes(t.E);
+    const size_t edge_smem = (size_t)sp_edge_bytes(t.E);
+    auto find = [&](bool rs) {
+        const IntVariant* f = nullptr;
+        for (const IntVariant& k : kInt)
+            if (k.bits == bits && k.dmax == dmax && k.rsmem == rs) f = &k;
+        return f;
+    };
+    auto ctas_per_sm = [&](const IntVariant* k, size_t bytes, int* out) -> cudaError_t {
+        cudaError_t e = allow_dynamic_smem((const void*)k->k, kSpMaxSmem + kSpEdgeSmem);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, (const void*)k->k, threads, bytes + edge_smem);
+        return e;
+    };
+    bool rsmem = false;
+    if (base + r_smem <= 160 * 1024) {
+        int per_s = 0, per_g = 0;
+        CUDA_TRY(ctas_per_sm(find(true), base + r_smem, &per_s));
+        CUDA_TRY(ctas_per_sm(find(false), base, &per_g));
+        rsmem = messages_in_smem(false, per_s, per_g);
+    }
+    const size_t payload = base + (rsmem ? r_smem : 0), smem = payload + edge_smem;
     if (payload > (size_t)kSpMaxSmem)
         return fail(LDPC_ERR_UNSUPPORTED, "int%d decoder: %zu B of shared memory", bits, payload);
-    const IntVariant* v = nullptr;
-    for (const IntVariant& k : kInt)
-        if (k.bits == bits && k.dmax == dmax && k.rsmem == rsmem) v = &k;
+    const IntVariant* v = find(rsmem);
     CUDA_TRY(allow_dynamic_smem((const void*)v->k, kSpMaxSmem + kSpEdgeSmem));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)v->k, threads, smem));

@@ -81,12 +81,6 @@ int setup_sp(ldpc_ctx* x) {
     // scratch E per thread
     const size_t r_smem = (size_t)(t.E | 1) * x->sp_threads * es;
     const size_t r_glob = (size_t)t.E * x->sp_threads * es;
-    // sum-product: messages in shared memory unless messages in global
-    // scratch (L2) give at least 1.5 times the CTAs per SM -- its tanh/atanh
-    // chains are latency-bound, so resident warps count for more than
-    // message latency, but one CTA more out of five does not pay for the L2
-    // round trips (802.11ad float: 6 vs 5 CTAs is 5 % slower).  Min-sum,
-    // light on arithmetic, keeps them in shared memory whenever they fit.
     auto find = [&](bool rs) {
         const SpVariant* f = nullptr;
         for (const SpVariant& k : kSp)
@@ -107,7 +101,7 @@ int setup_sp(ldpc_ctx* x) {
         int per_s = 0, per_g = 0;
         CUDA_TRY(ctas_per_sm(find(true), base_smem + r_smem, &per_s));
         CUDA_TRY(ctas_per_sm(find(false), base_smem, &per_g));
-        rsmem = !prod || 2 * per_g < 3 * per_s || getenv("LDPC_SP_RSMEM");
+        rsmem = messages_in_smem(prod, per_s, per_g) || getenv("LDPC_SP_RSMEM");
     }
     const SpVariant* v = find(rsmem);
     x->sp_kernel = dbl ? nullptr : v->k;

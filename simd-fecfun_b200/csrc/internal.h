@@ -63,6 +63,19 @@ inline long long spread_ctas(size_t n, long long slots, int sms) {
     return want > sms ? want : m < sms ? m : sms;
 }
 
+// Check messages of a float, double or integer decoder in shared memory (per_s
+// CTAs per SM) rather than in global scratch (L2, per_g CTAs per SM)?
+//   Sum-product: unless global messages give at least 1.5 times the CTAs.  Its
+// tanh/atanh chains are latency-bound, so resident warps count for more than
+// message latency, but one CTA more out of five does not pay for the L2 round
+// trips (802.11ad float 26.1e6 against 24.8e6 codewords/s).
+//   Min-sum: unless they give at least 2.5 times.  Light on arithmetic, it takes
+// that many more warps to cover the round trips (Mcw/s, shared against global:
+// float 802.11ad 63.7 / 53.8, 802.11n 2/3 Z = 81 14.1 / 13.7, 802.11ay 1/2
+// 16.9 / 23.9, 5G NR n6400 1.47 / 3.00; double 802.16e Z = 96 4.5 / 6.4,
+// 802.11ad 28.5 / 37.6).
+inline bool messages_in_smem(bool prod, int per_s, int per_g) { return 2 * per_g < (prod ? 3 : 5) * per_s; }
+
 // Arguments of one decode launch (device pointers).
 struct DecodeArgs {
     const void* llr = nullptr;
