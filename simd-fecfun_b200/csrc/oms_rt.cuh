@@ -295,11 +295,13 @@ struct RtTally {
 // Slot phase with the whole CTA on each finished codeword (used when the CTA
 // has more warps than codeword slots, where one warp per slot would leave the
 // others idle: 5G NR and other long codes).  Every thread derives the same
-// set of finished slots from shared state.  Element i of a codeword belongs to
-// thread i mod blockDim: that thread reads its finished posterior (hard bit,
-// error, posterior out) and then writes the next codeword's LLR there, so no
-// element is read by one thread and overwritten by another; warp w's lanes
+// set of finished slots from shared state.  Element i of a finished codeword is
+// read (hard bit, error, posterior out) by thread i mod blockDim; warp w's lanes
 // hold elements 32 (w + m nwarps) + lane, one hard-decision word per ballot.
+// With staging buffers that thread then writes the next codeword's LLR i there,
+// so no element is read by one thread and overwritten by another.  Without them
+// a thread loads four neighbouring LLRs at a time, over elements that others
+// read: all finished slots are read first, then, after a barrier, refilled.
 // Then, after a barrier, warp k mod nwarps does slot k's bookkeeping, claim
 // and prefetch.  Entered after a barrier that follows every thread's
 // cp.async wait; the caller commits the prefetches and ends with a barrier.
@@ -312,7 +314,7 @@ __device__ __forceinline__ void rt_slots_coop(const RtCode& C, const RtJob& job,
                                            unsigned long long (*s_cnt)[4], unsigned* s_err_bits, unsigned* s_err_slots) {
     const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, nwarps = nthr >> 5;
     const int n = C.n, z = C.z;
-    unsigned fin = 0;
+    unsigned fin = 0, refill = 0;   // slots, the same for every thread
     for (int k = 0; k < nslots; ++k) {
         if (s_cur[k] < 0) continue;
         if (!((s_synd[par][k >> sh] >> (8 * rt_byte(k, sh))) & 0x80u) || it_rd[k] + 1 >= C.max_iter) fin |= 1u << k;
@@ -348,8 +350,15 @@ __device__ __forceinline__ void rt_slots_coop(const RtCode& C, const RtJob& job,
         }
         if (job.post_out) rt_post(job.post_out + cw * (long long)n, pk, n, tid, nthr);
         if (s_next[k] >= 0) {
-            if (C.nostage) rt_fill_global(pk, job.llr + s_next[k] * (long long)n, n, tid, nthr);
+            if (C.nostage) refill |= 1u << k;
             else rt_fill(pk, stage_base + k * nstage, n, tid, nthr);
+        }
+    }
+    if (refill) {
+        __syncthreads();   // every warp has read the finished posteriors
+        for (unsigned f = refill; f; f &= f - 1) {
+            const int k = __ffs(f) - 1;
+            rt_fill_global(rt_slot(Ps, stride, k, sh), job.llr + s_next[k] * (long long)n, n, tid, nthr);
         }
     }
     // every thread has taken its decision from s_cur / it_rd / s_synd, summed
