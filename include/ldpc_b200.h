@@ -17,7 +17,8 @@
  *     bit i of a codeword (i < kbits = Z*(mcol-mrow)) is bit (i%32) of word
  *     i/32; each codeword takes hard_words = ceil(kbits/32) words.
  *   - A context is bound to one device and is not thread-safe; different
- *     contexts are independent.
+ *     contexts are independent.  Asynchronous decode calls of one context may
+ *     be given different streams and may overlap on the device.
  */
 #ifndef LDPC_B200_H
 #define LDPC_B200_H

@@ -245,6 +245,26 @@ void ldpc_code_destroy(ldpc_code* c) { delete c; }
 // ---------------------------------------------------------------------------
 namespace ldpc {
 
+int setup_areas(ldpc_ctx* x, int n) {
+    cudaFree(x->d_area_taken);
+    x->d_area_taken = nullptr;
+    x->n_areas = n;
+    if (!x->h_area_status) {
+        CUDA_TRY(cudaHostAlloc((void**)&x->h_area_status, sizeof(unsigned int), cudaHostAllocDefault));
+        *x->h_area_status = 0;
+    }
+    CUDA_TRY(cudaMalloc(&x->d_area_taken, (size_t)n * sizeof(unsigned int)));
+    CUDA_TRY(cudaMemset(x->d_area_taken, 0, (size_t)n * sizeof(unsigned int)));
+    CUDA_TRY(cudaStreamSynchronize(nullptr));   // the context's streams do not wait for the default one
+    return LDPC_OK;
+}
+
+int check_areas(const ldpc_ctx* x) {
+    if (x->h_area_status && *x->h_area_status)
+        return fail(LDPC_ERR_CUDA, "a decode launch of this context found no free message area; its outputs are incomplete");
+    return LDPC_OK;
+}
+
 int launch_decode(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     switch (x->cfg.variant) {
         case LDPC_INT8_OMS: return launch_oms(x, a, s);
@@ -405,6 +425,8 @@ void ldpc_ctx_destroy(ldpc_ctx* x) {
     cudaFree(x->d_rt_scratch);
     cudaFree(x->d_beta_tab);
     cudaFreeHost(x->h_small);
+    cudaFree(x->d_area_taken);
+    cudaFreeHost((void*)x->h_area_status);
     for (int i = 0; i < 2; ++i) {
         if (x->streams[i]) cudaStreamDestroy(x->streams[i]);
         for (int k = 0; k < 4; ++k) cudaFree(x->d_pipe[i][k]);
@@ -488,6 +510,7 @@ int decode_host_small(ldpc_ctx* x, const T* llr, size_t n, T* post, uint32_t* ha
     if (int rc = ldpc::launch_decode(x, a, s)) return rc;
     CUDA_TRY(cudaMemcpyAsync(h + at_post, dev + at_post, end - at_post, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaStreamSynchronize(s));
+    if (int rc = ldpc::check_areas(x)) return rc;
     if (post) memcpy(post, h + at_post, n * N * sizeof(T));
     if (hard) memcpy(hard, h + at_hard, n * HW * 4);
     if (iters) memcpy(iters, h + at_it, n);
@@ -554,6 +577,7 @@ int decode_host(ldpc_ctx* x, const T* llr, size_t n, T* post, uint32_t* hard, ui
         cudaError_t e = cudaStreamSynchronize(x->streams[b]);
         if (e != cudaSuccess && rc == LDPC_OK) rc = fail(LDPC_ERR_CUDA, "decode: %s", cudaGetErrorString(e));
     }
+    if (rc == LDPC_OK) rc = ldpc::check_areas(x);
     if (rc == LDPC_OK && tot_iter) {
         uint64_t s = 0;
         for (size_t i = 0; i < n; ++i) s += iters[i];

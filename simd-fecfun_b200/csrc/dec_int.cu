@@ -89,7 +89,10 @@ int setup_int(ldpc_ctx* x) {
     x->int_threads = threads;
     x->int_smem = (int)smem;
     x->int_ctas = per_sm * x->sms;
-    if (!rsmem) CUDA_TRY(cudaMalloc(&x->d_int_scratch, (size_t)x->int_ctas * r_glob));
+    if (!rsmem) {
+        CUDA_TRY(cudaMalloc(&x->d_int_scratch, (size_t)x->int_ctas * r_glob));
+        if (int rc = setup_areas(x, x->int_ctas)) return rc;
+    }
     // decode_row's offset and Max_row_simd in the element type (decode_functions.cpp:27-32, 59-62):
     // the float offset converts by truncation, the clamp is 1 - (CTYPE)max_row_metric for tiny values
     const double lim = bits == 16 ? 32767.0 : 2147483647.0;
@@ -105,6 +108,7 @@ int setup_int(ldpc_ctx* x) {
 int launch_int(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     if (!x->int_kernel) return fail(LDPC_ERR_INVALID_ARG, "context was not created for an int16/int32 decoder");
     if (a.n == 0) return LDPC_OK;
+    if (int rc = check_areas(x)) return rc;
     IntJob job;
     memset(&job, 0, sizeof(job));
     job.llr = a.llr;
@@ -122,6 +126,7 @@ int launch_int(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     job.beta = x->ibeta;
     job.maxv = x->imaxv;
     job.r_scratch = (int32_t*)x->d_int_scratch;
+    job.areas = areas_of(x);
     const long long want = spread_ctas(a.n, x->spt.G, x->sms);
     const int grid = (int)std::min<long long>(want, x->int_ctas);
     ((int_fn)x->int_kernel)<<<grid, x->int_threads, x->int_smem, s>>>(x->spt, job);

@@ -162,6 +162,7 @@ int setup_oms_rt(ldpc_ctx* x) {
     if (!rsmem) {
         x->rt_words_per_cta = (long long)E * threads;
         CUDA_TRY(cudaMalloc(&x->d_rt_scratch, (size_t)x->rt_ctas * x->rt_words_per_cta * 4));
+        if (int arc = setup_areas(x, x->rt_ctas)) return arc;
     }
     x->rt_kernel = k;
     x->rt_threads = threads;
@@ -173,6 +174,7 @@ int setup_oms_rt(ldpc_ctx* x) {
 
 int launch_oms_rt(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     if (a.n == 0) return LDPC_OK;
+    if (int rc = check_areas(x)) return rc;
     RtLaunch lp;
     memset(&lp, 0, sizeof(lp));
     lp.codes = x->d_rt_code;
@@ -189,6 +191,7 @@ int launch_oms_rt(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     j.n_buckets = std::max(1, std::min(a.n_buckets, OMS_MAX_BUCKETS));
     j.code = 0;
     lp.r_scratch = x->d_rt_scratch;
+    lp.areas = areas_of(x);
     lp.r_words_per_cta = x->rt_words_per_cta;
     lp.half = rt_half((double)a.n, (double)x->rt_G * x->rt_ctas);
     const long long want = spread_ctas(a.n, (lp.half ? 2LL : 4LL) * x->rt_G, x->sms);

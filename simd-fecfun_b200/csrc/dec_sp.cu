@@ -119,6 +119,7 @@ int setup_sp(ldpc_ctx* x) {
     x->sp_ctas = per_sm * x->sms;
     if (!rsmem) {
         CUDA_TRY(cudaMalloc(&x->d_sp_scratch, (size_t)x->sp_ctas * r_glob));
+        if (int rc = setup_areas(x, x->sp_ctas)) return rc;
     }
     // decode_row's Max_row_simd (decode_functions.cpp:27-32): 1 - (CTYPE)max_row_metric
     // below 1e-6 (sum-product), else max_row_metric, in the build's element type
@@ -149,6 +150,7 @@ SpJobT<T> sp_job(const ldpc_ctx* x, const DecodeArgs& a, T maxv) {
     job.beta = (T)x->cfg.beta;
     job.maxv = maxv;
     job.r_scratch = (T*)x->d_sp_scratch;
+    job.areas = areas_of(x);
     return job;
 }
 }  // namespace
@@ -156,6 +158,7 @@ SpJobT<T> sp_job(const ldpc_ctx* x, const DecodeArgs& a, T maxv) {
 int launch_sp(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s) {
     if (!x->sp_kernel && !x->sp64_kernel) return fail(LDPC_ERR_INVALID_ARG, "context was not created for a float decoder");
     if (a.n == 0) return LDPC_OK;
+    if (int rc = check_areas(x)) return rc;
     const long long want = spread_ctas(a.n, x->spt.G, x->sms);
     const int grid = (int)std::min<long long>(want, x->sp_ctas);
     if (x->sp64_kernel)

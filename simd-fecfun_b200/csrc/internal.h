@@ -158,6 +158,10 @@ struct ldpc_ctx {
     static constexpr int kQueues = 4;
     unsigned long long* d_queue = nullptr;      // work counters, one per concurrent launch
     unsigned int* d_status = nullptr;
+    // message areas in global memory (decoders whose messages are not in shared memory)
+    unsigned int* d_area_taken = nullptr;
+    int n_areas = 0;
+    volatile unsigned int* h_area_status = nullptr;   // page-locked; set by a launch that found no area
     unsigned long long* d_counters = nullptr;   // [OMS_MAX_BUCKETS][4] decode counters + [OMS_MAX_BUCKETS] uncoded
     cudaStream_t streams[2] = {nullptr, nullptr};
     // host-buffer pipeline: per stream, device buffers for one chunk (grow-only)
@@ -170,6 +174,11 @@ struct ldpc_ctx {
 };
 
 namespace ldpc {
+// n free message areas for the context's launches
+int setup_areas(ldpc_ctx* x, int n);
+inline MsgAreas areas_of(const ldpc_ctx* x) { return {x->d_area_taken, x->n_areas, (unsigned int*)x->h_area_status}; }
+// an error if a finished launch found no message area
+int check_areas(const ldpc_ctx* x);
 int setup_oms(ldpc_ctx* x);
 int launch_oms(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s);
 int setup_oms_rt(ldpc_ctx* x);

@@ -36,6 +36,7 @@ struct IntJob {
     int beta;                        // beta truncated to the element type
     int maxv;                        // Max_row_simd in the element type
     int32_t* r_scratch;              // global check messages when they do not fit shared memory
+    MsgAreas areas;                  //   and which CTA has which part of it
 };
 
 template <int W>
@@ -135,12 +136,15 @@ __global__ void __launch_bounds__(512) oms_int_kernel(const __grid_constant__ Sp
     const int t = tid / G, g = tid - (tid / G) * G;
     const bool active = t < z;
     const int gbase = g * stride;
+    __shared__ int s_area;
+    const int area = RSMEM ? 0 : take_area(job.areas, s_area);
+    if (area < 0) return;
     const SpEdge* edges = sp_load_edges(tb, sm_i);
     int32_t* Ps = sm_i + sp_edge_bytes(tb.E) / 4;
     TL* stage = reinterpret_cast<TL*>(Ps + ((G * stride + 3) & ~3));        // [G][nstage], 16-byte aligned
     const int nstage = ((n * (int)sizeof(TL) + 15) & ~15) / (int)sizeof(TL);
     int32_t* Rbase = RSMEM ? reinterpret_cast<int32_t*>(stage + G * nstage)
-                           : job.r_scratch + (long long)blockIdx.x * tb.E * nthr;
+                           : job.r_scratch + (long long)area * tb.E * nthr;
     // check messages: in shared memory each thread's E words are contiguous
     // at an odd stride (E | 1: a warp's lanes fall in distinct banks), so edge
     // e is the thread's base plus e; the global scratch keeps edge-major
@@ -280,6 +284,7 @@ __global__ void __launch_bounds__(512) oms_int_kernel(const __grid_constant__ Sp
             if (v) atomicAdd(job.counters + i, v);
         }
     }
+    if (!RSMEM) give_area(job.areas, s_area);
 }
 
 }  // namespace ldpc

@@ -36,6 +36,7 @@
 
 #include <type_traits>
 
+#include "msg_areas.cuh"
 #include "oms_f16.cuh"
 
 namespace ldpc {
@@ -437,6 +438,9 @@ __global__ void __launch_bounds__(512) oms_rt_kernel(const __grid_constant__ RtL
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int warp = tid >> 5, lane = tid & 31, nwarps = nthr >> 5;
     const RtConst kc(lp.zero);
+    __shared__ int s_area;
+    const int area = RSMEM ? 0 : take_area(lp.areas, s_area);
+    if (area < 0) return;
     if (tid == 0) s_code_idx = -1;
 
     const int n_chunks = lp.jobs ? lp.n_chunks : (int)gridDim.x;
@@ -489,7 +493,7 @@ __global__ void __launch_bounds__(512) oms_rt_kernel(const __grid_constant__ RtL
         // scratch keeps edge-major words (coalesced)
         const int rstride = RSMEM ? 1 : nthr;
         uint32_t* const Rt = RSMEM ? reinterpret_cast<uint32_t*>(stage_base + nslots * nstage) + tid * (E | 1)
-                                   : lp.r_scratch + (long long)blockIdx.x * lp.r_words_per_cta + tid;
+                                   : lp.r_scratch + (long long)area * lp.r_words_per_cta + tid;
 
         for (int i = tid; i < OMS_MAX_BUCKETS * 4; i += nthr) (&s_cnt[0][0])[i] = 0;
         for (int i = tid; i < G * stride; i += nthr) Ps[i] = 0x80808080u;   // P = 0
@@ -648,6 +652,7 @@ __global__ void __launch_bounds__(512) oms_rt_kernel(const __grid_constant__ RtL
             }
         }
     }
+    if (!RSMEM) give_area(lp.areas, s_area);
 }
 
 }  // namespace ldpc

@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "gen_trees.cuh"
+#include "msg_areas.cuh"
 #include "sp_math.cuh"
 #include "tables.h"
 #include "writeout.cuh"
@@ -343,8 +344,12 @@ __global__ void __maxnreg__(sp_max_regs(DMAX, PROD, RSMEM)) sp_f32_kernel(const 
     extern __shared__ __align__(16) float sm_f[];
     const long long lo = job.ncw * blockIdx.x / gridDim.x, hi = job.ncw * (blockIdx.x + 1) / gridDim.x;
     const SpEdge* edges = sp_load_edges(tb, sm_f);
+    __shared__ int s_area;
+    const int area = RSMEM ? 0 : take_area(job.areas, s_area);
+    if (area < 0) return;
     sp_decode_range<DMAX, PROD, RSMEM>(tb, edges, job, lo, hi, sm_f + sp_edge_bytes(tb.E) / 4,
-                                       RSMEM ? nullptr : job.r_scratch + (long long)blockIdx.x * tb.E * blockDim.x);
+                                       RSMEM ? nullptr : job.r_scratch + (long long)area * tb.E * blockDim.x);
+    if (!RSMEM) give_area(job.areas, s_area);
 }
 
 template <int DMAX, bool PROD, bool RSMEM, int MAXT>
@@ -353,8 +358,12 @@ __global__ void __launch_bounds__(MAXT) sp_f64_kernel(const __grid_constant__ Sp
     extern __shared__ __align__(16) double sm_d[];
     const long long lo = job.ncw * blockIdx.x / gridDim.x, hi = job.ncw * (blockIdx.x + 1) / gridDim.x;
     const SpEdge* edges = sp_load_edges(tb, sm_d);
+    __shared__ int s_area;
+    const int area = RSMEM ? 0 : take_area(job.areas, s_area);
+    if (area < 0) return;
     sp_decode_range<DMAX, PROD, RSMEM>(tb, edges, job, lo, hi, sm_d + sp_edge_bytes(tb.E) / 8,
-                                       RSMEM ? nullptr : job.r_scratch + (long long)blockIdx.x * tb.E * blockDim.x);
+                                       RSMEM ? nullptr : job.r_scratch + (long long)area * tb.E * blockDim.x);
+    if (!RSMEM) give_area(job.areas, s_area);
 }
 
 }  // namespace ldpc

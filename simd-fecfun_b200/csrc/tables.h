@@ -62,6 +62,13 @@ struct SpTables {
     SpEdge edge[SP_MAX_E];
 };
 
+// Message areas of a context in global memory (msg_areas.cuh).
+struct MsgAreas {
+    unsigned int* taken;             // [n] 1: a running CTA has the area; null: area = block index
+    int n;                           // CTAs that can be resident at a time
+    unsigned int* status;            // set to 1 when a CTA found no area (page-locked host memory)
+};
+
 template <class T>                   // T = float or double
 struct SpJobT {
     const T* llr;
@@ -80,6 +87,7 @@ struct SpJobT {
     T beta;
     T maxv;                          // Max_val as decode_row computes it
     T* r_scratch;                    // global check messages when they do not fit shared memory
+    MsgAreas areas;                  //   and which CTA has which part of it
 };
 using SpJob = SpJobT<float>;
 
@@ -138,6 +146,7 @@ struct RtLaunch {
     RtJob job0;
     uint32_t* r_scratch;             // check messages in global memory (when not in shared memory)
     long long r_words_per_cta;
+    MsgAreas areas;                  // single-code launches: which CTA has which part of it
     uint32_t zero;                   // 0 (RtConst)
     int half;                        // 1: two codewords per word (bytes 0 and 1), 2G slots; 0: four, 4G slots
 };
