@@ -260,3 +260,26 @@ def test_wide_outputs_are_the_float_llrs(capi, bits, name, n, offset):
     assert torch.equal(got, want)
     assert (w[:offset] == 77).all() and (w[offset + f.numel():] == 77).all()
     assert torch.equal(uf, uw)
+
+
+@pytest.mark.parametrize("offset", [0, 4, 8, 1])
+@pytest.mark.parametrize("name", ["16e 1/2", "11ad 1/2"])
+@pytest.mark.parametrize("z", [1, 2, 3, 5, 8, 31, 32, 33])
+def test_encode_narrow_columns(capi, oracle, z, name, offset):
+    """Columns narrower than a store (down to one bit), one word wide, and one
+    bit more; N = 24 Z and 16 Z: 16- and 8-byte stores, 4- and 1-byte ones by
+    the output's offset."""
+    import torch
+    from conftest import pack_bits
+    from ldpc_b200 import codes
+    code = codes.make_code(name, z_over=z)
+    ctx = capi.Context(capi.Code.from_tables(code), variant=capi.LDPC_F32_OMS, max_iter=2)
+    rng = np.random.default_rng(z)
+    for n in (1, 45, 3000):
+        info = rng.integers(0, 2, (n, (code.mcol - code.mrow) * code.z), dtype=np.uint8)
+        data = torch.from_numpy(pack_bits(info).view(np.int32)).cuda()
+        out = torch.full((n * code.n + 32,), 7, dtype=torch.uint8, device="cuda")
+        ctx.encode(data, n, out.data_ptr() + offset)
+        got = out.cpu().numpy()
+        assert np.array_equal(got[offset:offset + n * code.n].reshape(n, code.n), oracle.encode(code, info))
+        assert (got[:offset] == 7).all() and (got[offset + n * code.n:] == 7).all()
