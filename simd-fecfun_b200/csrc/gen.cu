@@ -60,7 +60,7 @@ EncodeShape encode_shape(const GenTables& t, long long n, int sms, int* smem) {
     s.stride = words + (((zw - words) % 32) + 32) % 32;
     s.cws = std::max(1, std::min(32 / zw, 56 * 1024 / (8 * 4 * s.stride)));
     while (s.cws > 1 && n < (long long)s.cws * 8 * sms) s.cws = (s.cws + 1) / 2;
-    s.inv_z = t.z > 1 ? (uint32_t)(((1ull << 32) + t.z - 1) / t.z) : 0u;
+    s.inv_z = (uint32_t)(((1ull << 31) + t.z - 1) / t.z);
     *smem = 8 * 4 * s.cws * s.stride;
     return s;
 }

@@ -600,7 +600,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
 // 802.16e 1/2 Z = 96, 65536 codewords (160 MB in and out): 572 -> 76 us.
 struct EncodeShape {
     int cws, stride;                 // codewords per warp, words per codeword in shared memory
-    uint32_t inv_z;                  // ceil(2^32 / z): c = umulhi(i, inv_z) for i < 2^20; 0 for z = 1 (c = i)
+    uint32_t inv_z;                  // ceil(2^31 / z), 32 bits for z = 1 too: c = umulhi(2 i, inv_z) for i < 2^20
 };
 
 // cols: column c's words at [c * (zw + 1)], a zero word behind them; the data
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(256) encode_kernel(const __grid_constant__ Gen
                 q -= nv;
                 ++c;
             }
-            const int idx = V * q, col = sh.inv_z ? (int)__umulhi((uint32_t)idx, sh.inv_z) : idx, p = idx - col * z;
+            const int idx = V * q, col = (int)__umulhi(2u * (uint32_t)idx, sh.inv_z), p = idx - col * z;
             const uint32_t* w = mine + c * sh.stride + col * (zw + 1);
             uint32_t v = stream_bits32(w, p);
             for (int have = z - p; have < V; have += z) {
