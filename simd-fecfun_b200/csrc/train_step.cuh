@@ -16,9 +16,11 @@
 // codeword, written once and read once in the opposite order (so that L2
 // serves the younger part), against 384 KB of posteriors and messages written
 // to checkpoints, read back, and the layers recomputed from them.  65536
-// codewords: 105 ms (13 forward, 84 adjoint, 8 for the loss in torch) -> 18.7 ms;
+// codewords: 105 ms (13 forward, 84 adjoint, 8 for the loss in torch) -> 19.3 ms;
 // issue 58 %, DRAM 29 %, 15 warps per SM (shared memory).  Q loaded one row
-// ahead: 25.4 -> 22.6 ms; sent bits in shared memory: -> 18.7 ms.
+// ahead: 25.4 -> 22.6 ms; sent bits in shared memory: -> 18.8 ms; the loss in full
+// float precision (expf, the product of 1 + e^-|x| kept less 1, a quotient with
+// residual step): -> 19.3 ms.
 //
 // Layout: G codewords per CTA, thread (g, t) = check row t of every layer of
 // codeword g, as the decoders.  The messages R (forward) and their adjoint
@@ -209,25 +211,28 @@ __global__ void __launch_bounds__(NT) oms_train_step(const __grid_constant__ SpT
                 __syncthreads();
             }
             // loss softplus(x), x = -s P: max(x, 0) + ln(1 + e^-|x|), the logarithms of up to 32
-            // elements as one of their product; its adjoint is -s times the logistic of x
+            // elements as one of their product.  The product is kept less 1, a sum of positive
+            // terms, so that small e^-|x| count in full (a converged batch has no others; as a
+            // product of rounded 1 + e^-|x| its loss was 1 % off at |P| = 12, 0 beyond 16.6).  The
+            // adjoint is -s times the logistic of x.
             if (active) {
                 const float w = __ldg(job.loss_w + it), wk = w * job.inv_norm;
                 float* gs = GRAD ? Gs + (long long)it * mcol * NT : nullptr;
                 float sum = 0.0f;
                 for (int b = 0; b < mcol; b += 32) {
                     const int bn = min(32, mcol - b);
-                    float prod = 1.0f;
+                    float prod1 = 0.0f;   // product - 1
                     uint32_t m = ~sent[(b >> 5) * blockDim.x];
 #pragma unroll 8
                     for (int c = 0; c < bn; ++c, m >>= 1) {
                         const uint32_t sg = m << 31;
                         const float x = sp_flip(Pg[(b + c) * z + t], sg);
-                        const float ex = __expf(-fabsf(x)), u = 1.0f + ex;
+                        const float ex = expf(-fabsf(x));
                         sum += fmaxf(x, 0.0f);
-                        prod *= u;
-                        if (GRAD) gs[(b + c) * NT] = sp_flip(wk * __fdividef(x < 0.0f ? ex : 1.0f, u), sg);
+                        prod1 = __fmaf_rn(prod1, ex, prod1) + ex;
+                        if (GRAD) gs[(b + c) * NT] = sp_flip(wk * spm_div(x < 0.0f ? ex : 1.0f, 1.0f + ex), sg);
                     }
-                    sum += logf(prod);
+                    sum += log1pf(prod1);
                 }
                 loss += (double)w * (double)sum;
             }

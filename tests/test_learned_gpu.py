@@ -202,3 +202,34 @@ def test_loss_kernel_matches_checkpointed_kernels(capi, name, z, n):
     ref = part.double().sum(dim=0).view(iters, L)
     assert abs(loss.item() - want.item()) <= 1e-6 * want.item()
     assert (beta.grad.double() - ref).norm() <= 1e-5 * ref.norm()
+
+
+def test_loss_of_a_converged_batch(capi):
+    """Every posterior right and of magnitude 12..27: each term ln(1 + e^-|P|)
+    is 1e-5 or less.  Against softplus in double of the same float posteriors;
+    per term one exponential (2 ulp) and two roundings of a sum of positive
+    terms, at most 32 in a row, then one logarithm (2 ulp): 70 x 2^-24 at most,
+    1e-5 allowed, relative."""
+    import torch
+    import torch.nn.functional as F
+    from ldpc_b200 import codes, learned
+    code = codes.make_code("16e 1/2", z_over=24)
+    ctx = _ctx(capi, code, mrm=0.25)
+    n, iters, N = 50, 3, code.n
+    g = torch.Generator(device="cuda").manual_seed(1)
+    info = torch.randint(-2 ** 31, 2 ** 31, (n, ctx.info.hard_words), dtype=torch.int32, generator=g, device="cuda")
+    bits = torch.empty((n, N), dtype=torch.uint8, device="cuda")
+    ctx.encode(info, n, bits)
+    for lo, hi in ((12.0, 25.0), (16.7, 25.0)):
+        llr = (1.0 - 2.0 * bits.float()) * (lo + (hi - lo) * torch.rand((n, N), generator=g, device="cuda"))
+        beta = torch.full((iters, code.mrow), 0.5, device="cuda")
+        w = torch.tensor([1.0, 0.5, 2.0], device="cuda")
+        loss = learned.LearnedOMSLoss.apply(beta, llr, bits, w, ctx)
+        ckpt_p = torch.empty((iters + 1, n, N), device="cuda")
+        ckpt_r = torch.empty((iters, n, ctx.info.edges), device="cuda")
+        capi.check(capi.lib.ldpc_learned_forward(ctx.h, llr.data_ptr(), n, iters, beta.data_ptr(), ckpt_p.data_ptr(),
+                                                 ckpt_r.data_ptr(), None))
+        x = -(1.0 - 2.0 * bits.double()) * ckpt_p[1:].double()
+        assert x.max() < -12.0 and x.min() > -27.0
+        want = (w.double() * torch.log1p(torch.exp(x)).sum(dim=(1, 2))).sum() / (n * N)
+        assert abs(loss.item() - want.item()) <= 1e-5 * want.item()
