@@ -302,7 +302,9 @@ int ldpc_learned_backward(ldpc_ctx *ctx, size_t n, int iters, const float *beta,
  * [grad_rows][iters*mrow] (column sums = dL/dbeta) and scratch
  * [scratch_floats]; gbeta_part = scratch = NULL: the loss alone.  All partial
  * sums are in a fixed order.  Takes the codes that ldpc_learned_backward
- * (with the gradient) or ldpc_learned_forward (without) takes. */
+ * (with the gradient) or ldpc_learned_forward (without) takes, if the messages
+ * of Z rounded up to a multiple of 32 fit shared memory; LDPC_ERR_UNSUPPORTED
+ * otherwise (LearnedOMSLoss then runs those two). */
 int ldpc_learned_loss_size(ldpc_ctx *ctx, size_t n, int iters, int want_grad, int *loss_rows, int *grad_rows,
                            size_t *scratch_floats);
 int ldpc_learned_loss(ldpc_ctx *ctx, const float *llr, const uint8_t *cw_bits, size_t n, int iters,

@@ -2,7 +2,8 @@
 
 * :class:`LearnedOMSLoss` -- ``torch.autograd.Function`` over one CUDA kernel
   that unrolls the decoder, evaluates the loss and runs the hand-written
-  adjoint (``ldpc_learned_loss``).
+  adjoint (``ldpc_learned_loss``); codes that it does not hold go through the
+  checkpointing kernels (``ldpc_learned_forward`` / ``ldpc_learned_backward``).
 * :func:`reference_loss` -- the same unrolled decoder and loss written with
   differentiable torch operations (any dtype, CPU or GPU): the reference
   gradient for the adjoint, and the function the finite-difference checks
@@ -60,8 +61,10 @@ class LearnedOMSLoss(torch.autograd.Function):
                 raise RuntimeError("LearnedOMSLoss needs its tensors on one CUDA device")
         inv_norm = 1.0 / float(n * N) if n * N else float("nan")
         rows, grows, words = C.c_int(), C.c_int(), C.c_size_t()
-        capi.check(capi.lib.ldpc_learned_loss_size(ctx.h, n, iters, int(grad), C.byref(rows), C.byref(grows),
-                                                   C.byref(words)))
+        rc = capi.lib.ldpc_learned_loss_size(ctx.h, n, iters, int(grad), C.byref(rows), C.byref(grows), C.byref(words))
+        if rc == capi.LDPC_ERR_UNSUPPORTED:
+            return LearnedOMSLoss._checkpointed(fctx, beta, llr, cw_bits, loss_w, ctx)
+        capi.check(rc)
         loss = torch.empty(rows.value, dtype=torch.float64, device=llr.device)
         part = scratch = None
         if grad:
@@ -73,11 +76,42 @@ class LearnedOMSLoss(torch.autograd.Function):
         # the gradient is at hand already; the inputs are saved so that autograd
         # still sees one changed in place before backward
         fctx.save_for_backward(beta, cw_bits, loss_w, part.sum(dim=0).view(iters, L) if grad else None)
+        fctx.ctx = None
         return loss.sum().float()
 
     @staticmethod
+    def _checkpointed(fctx, beta, llr, cw_bits, loss_w, ctx):
+        """Codes that the one-launch kernel does not hold (messages of Z rounded
+        up to whole warps, or a gradient wanted where no adjoint fits): the loss
+        from the forward kernel's checkpoints, the gradient, if there is one to
+        be had, from the adjoint kernel."""
+        iters = beta.shape[0]
+        n, N = llr.shape
+        ckpt_p = torch.empty((iters + 1, n, N), dtype=torch.float32, device=llr.device)
+        ckpt_r = torch.empty((iters, n, ctx.info.edges), dtype=torch.float32, device=llr.device)
+        capi.check(capi.lib.ldpc_learned_forward(ctx.h, llr.data_ptr(), n, iters, beta.data_ptr(), ckpt_p.data_ptr(),
+                                                 ckpt_r.data_ptr(), _stream()))
+        s = 1.0 - 2.0 * cw_bits.float()
+        per_it = F.softplus(-s.unsqueeze(0) * ckpt_p[1:]).sum(dim=(1, 2))
+        fctx.save_for_backward(beta, cw_bits, loss_w, ckpt_p, ckpt_r)
+        fctx.ctx = ctx
+        return (loss_w * per_it).sum() / float(n * N)
+
+    @staticmethod
     def backward(fctx, g):
-        gbeta = fctx.saved_tensors[3]
+        if fctx.ctx is None:
+            gbeta = fctx.saved_tensors[3]
+        else:
+            beta, cw_bits, loss_w, ckpt_p, ckpt_r = fctx.saved_tensors
+            iters, L = beta.shape
+            n, N = cw_bits.shape
+            grid = C.c_int()
+            capi.check(capi.lib.ldpc_learned_grid(fctx.ctx.h, n, C.byref(grid)))
+            part = torch.empty((grid.value, iters * L), dtype=torch.float32, device=beta.device)
+            capi.check(capi.lib.ldpc_learned_backward(fctx.ctx.h, n, iters, beta.data_ptr(), ckpt_p.data_ptr(),
+                                                      ckpt_r.data_ptr(), cw_bits.data_ptr(), loss_w.data_ptr(),
+                                                      1.0 / float(n * N), part.data_ptr(), None, _stream()))
+            gbeta = part.sum(dim=0).view(iters, L)
         return gbeta * g if gbeta is not None else None, None, None, None, None
 
 

@@ -233,3 +233,30 @@ def test_loss_of_a_converged_batch(capi):
         assert x.max() < -12.0 and x.min() > -27.0
         want = (w.double() * torch.log1p(torch.exp(x)).sum(dim=(1, 2))).sum() / (n * N)
         assert abs(loss.item() - want.item()) <= 1e-5 * want.item()
+
+
+# the messages of Z = 176 rounded up to 192 rows leave no room for the first one's posteriors;
+# the second one's loss fits, its adjoint does not
+@pytest.mark.parametrize("name", ["5GNR_n9443_k3872", "5GNR_n8604_k3872"])
+def test_loss_of_codes_without_an_adjoint(capi, name):
+    """Codes that the decoder holds but the adjoint does not: the loss, with
+    and without a gradient wanted, and an error from backward."""
+    import torch
+    from ldpc_b200 import codes, learned
+    code = codes.code_by_name(name)
+    ctx = _ctx(capi, code)
+    n, iters = 6, 3
+    g = torch.Generator(device="cuda").manual_seed(3)
+    llr = 2.0 + 3.0 * torch.randn((n, code.n), generator=g, device="cuda")
+    bits = (torch.rand((n, code.n), generator=g, device="cuda") < 0.1).to(torch.uint8)
+    beta = torch.full((iters, code.mrow), 0.5, device="cuda")
+    w = torch.tensor([1.0, 0.5, 2.0], device="cuda")
+    want = float(learned.reference_loss(code, beta.double(), llr.double(), bits, w.double(), 20.0,
+                                        [t.cuda() for t in learned.layer_tables(code)]))
+    alone = learned.LearnedOMSLoss.apply(beta, llr, bits, w, ctx)
+    assert abs(alone.item() - want) <= 1e-4 * want
+    beta.requires_grad_(True)
+    loss = learned.LearnedOMSLoss.apply(beta, llr, bits, w, ctx)
+    assert abs(loss.item() - want) <= 1e-4 * want
+    with pytest.raises(capi.LdpcError):
+        loss.backward()
