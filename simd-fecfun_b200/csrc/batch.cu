@@ -201,7 +201,7 @@ int float_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int thread
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, threads, smem));
     if (per_sm < 1) return fail(LDPC_ERR_UNSUPPORTED, "batch plan: %d threads x %zu B do not fit an SM", threads, smem);
-    const long long ctas = (long long)per_sm * b->sms;
+    const long long ctas = ldpc::launch_ctas(per_sm * b->sms);
     std::vector<ldpc::SpCode> hc(nc);
     for (int c = 0; c < nc; ++c) {
         memset(&hc[c], 0, sizeof(hc[c]));
@@ -307,7 +307,7 @@ int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)p->k, threads, smem));
     if (per_sm < 1) return fail(LDPC_ERR_UNSUPPORTED, "batch plan: %d threads x %zu B do not fit an SM", threads, smem);
-    const long long ctas = (long long)per_sm * b->sms;
+    const long long ctas = ldpc::launch_ctas(per_sm * b->sms);
 
     std::vector<ldpc::RtCode> hc(nc);
     for (int c = 0; c < nc; ++c) {

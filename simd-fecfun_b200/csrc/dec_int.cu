@@ -88,10 +88,11 @@ int setup_int(ldpc_ctx* x) {
     x->int_kernel = (void*)v->k;
     x->int_threads = threads;
     x->int_smem = (int)smem;
-    x->int_ctas = per_sm * x->sms;
+    const int resident = per_sm * x->sms;
+    x->int_ctas = launch_ctas(resident);
     if (!rsmem) {
-        CUDA_TRY(cudaMalloc(&x->d_int_scratch, (size_t)x->int_ctas * r_glob));
-        if (int rc = setup_areas(x, x->int_ctas)) return rc;
+        CUDA_TRY(cudaMalloc(&x->d_int_scratch, (size_t)resident * r_glob));
+        if (int rc = setup_areas(x, resident)) return rc;
     }
     // decode_row's offset and Max_row_simd in the element type (decode_functions.cpp:27-32, 59-62):
     // the float offset converts by truncation, the clamp is 1 - (CTYPE)max_row_metric for tiny values

@@ -161,7 +161,7 @@ int setup_oms(ldpc_ctx* x) {
     if (per_sm < 1)
         return fail(LDPC_ERR_UNSUPPORTED, "int8 decoder: %d threads x %d B shared memory do not fit an SM",
                     x->oms_threads, x->oms_smem);
-    x->oms_ctas = per_sm * x->sms;
+    x->oms_ctas = launch_ctas(per_sm * x->sms);
     return LDPC_OK;
 }
 

@@ -156,13 +156,14 @@ int setup_oms_rt(ldpc_ctx* x) {
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, threads, smem));
     if (per_sm < 1) return fail(LDPC_ERR_UNSUPPORTED, "int8 decoder: %d threads x %zu B do not fit an SM", threads, smem);
-    x->rt_ctas = per_sm * x->sms;
+    const int resident = per_sm * x->sms;
+    x->rt_ctas = launch_ctas(resident);
     CUDA_TRY(cudaMalloc(&x->d_rt_code, sizeof(RtCode)));
     CUDA_TRY(cudaMemcpy(x->d_rt_code, &host, sizeof(RtCode), cudaMemcpyHostToDevice));
     if (!rsmem) {
         x->rt_words_per_cta = (long long)E * threads;
-        CUDA_TRY(cudaMalloc(&x->d_rt_scratch, (size_t)x->rt_ctas * x->rt_words_per_cta * 4));
-        if (int arc = setup_areas(x, x->rt_ctas)) return arc;
+        CUDA_TRY(cudaMalloc(&x->d_rt_scratch, (size_t)resident * x->rt_words_per_cta * 4));
+        if (int arc = setup_areas(x, resident)) return arc;
     }
     x->rt_kernel = k;
     x->rt_threads = threads;

@@ -116,10 +116,11 @@ int setup_sp(ldpc_ctx* x) {
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, x->sp_threads, x->sp_smem));
     if (per_sm < 1) return fail(LDPC_ERR_UNSUPPORTED, "float decoder: launch does not fit an SM");
-    x->sp_ctas = per_sm * x->sms;
+    const int resident = per_sm * x->sms;
+    x->sp_ctas = launch_ctas(resident);
     if (!rsmem) {
-        CUDA_TRY(cudaMalloc(&x->d_sp_scratch, (size_t)x->sp_ctas * r_glob));
-        if (int rc = setup_areas(x, x->sp_ctas)) return rc;
+        CUDA_TRY(cudaMalloc(&x->d_sp_scratch, (size_t)resident * r_glob));
+        if (int rc = setup_areas(x, resident)) return rc;
     }
     // decode_row's Max_row_simd (decode_functions.cpp:27-32): 1 - (CTYPE)max_row_metric
     // below 1e-6 (sum-product), else max_row_metric, in the build's element type

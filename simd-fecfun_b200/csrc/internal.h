@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -75,6 +76,15 @@ inline long long spread_ctas(size_t n, long long slots, int sms) {
 // 16.9 / 23.9, 5G NR n6400 1.47 / 3.00; double 802.16e Z = 96 4.5 / 6.4,
 // 802.11ad 28.5 / 37.6).
 inline bool messages_in_smem(bool prod, int per_s, int per_g) { return 2 * per_g < (prod ? 3 : 5) * per_s; }
+
+// CTAs that a context's or plan's launches may have: all that the device holds,
+// or LDPC_MAX_CTAS (read when the context or plan is created).  With few CTAs a
+// small call fills every slot of a CTA and refills it, which otherwise takes
+// thousands of codewords.
+inline int launch_ctas(int resident) {
+    const char* e = getenv("LDPC_MAX_CTAS");
+    return e && atoi(e) > 0 && atoi(e) < resident ? atoi(e) : resident;
+}
 
 // Arguments of one decode launch (device pointers).
 struct DecodeArgs {

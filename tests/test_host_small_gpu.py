@@ -32,3 +32,38 @@ def test_small_and_large_host_calls(capi, oracle, n, outputs):
         if hard is not None:
             bits = np.unpackbits(hard.view(np.uint8), axis=1, bitorder="little")[:, :336]
             assert np.array_equal(bits, (post_o[:, :336] < 0).astype(np.uint8))
+
+
+@pytest.mark.parametrize("kind", ["int16", "int32", "f32", "f64"])
+@pytest.mark.parametrize("outputs", ["phi", "i", ""])
+def test_small_host_calls_of_wider_types(capi, kind, outputs):
+    """Either side of 256 KB for each element type, against the same LLRs
+    decoded from device memory."""
+    import torch
+    from ldpc_b200 import codes
+    code = codes.make_code("11ad 1/2")
+    variant, dt, clamp, beta = {"int16": (capi.LDPC_INT16_OMS, torch.int16, 31.0, 1.0),
+                                "int32": (capi.LDPC_INT32_OMS, torch.int32, 31.0, 1.0),
+                                "f32": (capi.LDPC_F32_SP, torch.float32, 6e-8, 0.0),
+                                "f64": (capi.LDPC_F64_OMS, torch.float64, 31.0, 0.5)}[kind]
+    ctx = capi.Context(capi.Code.from_tables(code), variant=variant, max_iter=10, max_row_metric=clamp, beta=beta,
+                       llr_scale=2.0, max_abs_llr=24.0)
+    es = torch.empty(0, dtype=dt).element_size()
+    limit = (262144 - 1024) // (code.n * es * (2 if "p" in outputs else 1) + (44 if "h" in outputs else 0) + 1)
+    for n in (1, 17, limit - 1, limit, limit + 1):
+        llr = torch.empty((1, n, code.n), dtype=dt, device="cuda")
+        ctx.generate(n, 0, [-0.75], n, **({"llr_f32": llr} if kind == "f32" else {"llr_int": llr}))
+        p, it = torch.empty_like(llr), torch.empty(n, dtype=torch.uint8, device="cuda")
+        h = torch.empty((n, 11), dtype=torch.int32, device="cuda")
+        getattr(ctx, "decode_" + kind)(llr, n, post=p, hard=h, iters=it)
+        host = llr.cpu().numpy()
+        post = np.zeros_like(host) if "p" in outputs else None
+        hard = np.zeros((n, 11), np.int32) if "h" in outputs else None
+        iters = np.zeros(n, np.uint8) if "i" in outputs else None
+        tot = C.c_uint64()
+        capi.check(getattr(capi.lib, "ldpc_decode_%s_host" % kind)(ctx.h, host.ctypes.data, n, capi._ptr(post),
+                                                                   capi._ptr(hard), capi._ptr(iters), C.byref(tot)))
+        assert tot.value == int(it.sum(dtype=torch.int64))
+        assert post is None or np.array_equal(post.view(np.uint8), p.cpu().numpy().view(np.uint8))
+        assert hard is None or np.array_equal(hard, h.cpu().numpy())
+        assert iters is None or np.array_equal(iters, it.cpu().numpy())
