@@ -277,7 +277,7 @@ int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads
     for (int i = 0; i < n_jobs; ++i) used[jobs[i].code] = 1;
     std::vector<int> G(nc, 1);
     int dmax = 8, maxE = 0;
-    bool quirk = false, rsmem = true;
+    bool quirk = false, rsmem = true, exact = true;
     for (int c = 0; c < nc; ++c) {
         if (!used[c]) continue;
         const ldpc_code& cd = b->codes[c];
@@ -288,6 +288,7 @@ int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads
             return fail(LDPC_ERR_UNSUPPORTED, "batch plan: code %d (N=%d) does not fit shared memory", c, n);
         if (ldpc::rt_smem_bytes(n, G[c], E, threads, true) > (size_t)ldpc::kRtMaxSmem) rsmem = false;
         dmax = std::max(dmax, ldpc::rt_dmax(cd.max_row_weight));
+        exact = exact && ldpc::rt_exact(cd);
         maxE = std::max(maxE, E);
         for (int v : b->beta8[c]) quirk |= v == 0;
         for (int v : b->tab8[c]) quirk |= v == 0;
@@ -300,7 +301,7 @@ int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads
     }
     std::unique_ptr<ldpc_batch_plan, PlanDel> p(new ldpc_batch_plan);
     p->device = b->device;
-    p->k = ldpc::rt_kernel_for(dmax, quirk, rsmem);
+    p->k = ldpc::rt_kernel_for(dmax, exact, quirk, rsmem);
     p->threads = threads;
     p->smem = (int)smem;
     CUDA_TRY(ldpc::allow_dynamic_smem((const void*)p->k, ldpc::kRtMaxSmem));
@@ -312,7 +313,7 @@ int int8_plan(ldpc_batch* b, const ldpc_batch_job* jobs, int n_jobs, int threads
     std::vector<ldpc::RtCode> hc(nc);
     for (int c = 0; c < nc; ++c) {
         const ldpc_code& cd = b->codes[c];
-        if (int rc = ldpc::make_rt_code(cd, (int)b->cfgs[c].max_iter, b->maxv2[c], b->beta8[c].data(), 0, G[c], &hc[c]))
+        if (int rc = ldpc::make_rt_code(cd, (int)b->cfgs[c].max_iter, b->maxv2[c], b->beta8[c].data(), 0, G[c], exact, &hc[c]))
             return rc;
     }
     // offset tables of the used codes, one device buffer
@@ -428,7 +429,7 @@ int int8_class(const ldpc_batch* b, int c, int threads, PlanClass* out) {
     for (int v : b->beta8[c]) quirk |= v == 0;
     for (int v : b->tab8[c]) quirk |= v == 0;
     const int dmax = ldpc::rt_dmax(cd.max_row_weight);
-    ldpc::rt_fn k = ldpc::rt_kernel_for(dmax, quirk, rsmem);
+    ldpc::rt_fn k = ldpc::rt_kernel_for(dmax, ldpc::rt_exact(cd), quirk, rsmem);
     CUDA_TRY(ldpc::allow_dynamic_smem((const void*)k, ldpc::kRtMaxSmem));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, threads,

@@ -14,20 +14,41 @@ namespace ldpc {
 namespace {
 struct RtVariant {
     int dmax;
-    bool quirk, rsmem;
+    bool exact, quirk, rsmem;
     rt_fn k;
 };
-#define RTV(D_) {D_, false, false, oms_rt_kernel<D_, false, false>}, {D_, false, true, oms_rt_kernel<D_, false, true>}, \
-                {D_, true, false, oms_rt_kernel<D_, true, false>},   {D_, true, true, oms_rt_kernel<D_, true, true>}
-const RtVariant kRt[] = {RTV(8), RTV(12), RTV(16), RTV(24), RTV(32)};
+#define RTV(D_, X_)                                                                                             \
+    {D_, X_, false, false, oms_rt_kernel<D_, X_, false, false>}, {D_, X_, false, true, oms_rt_kernel<D_, X_, false, true>}, \
+    {D_, X_, true, false, oms_rt_kernel<D_, X_, true, false>},   {D_, X_, true, true, oms_rt_kernel<D_, X_, true, true>}
+const RtVariant kRt[] = {RTV(8, true),   RTV(8, false),  RTV(12, true), RTV(12, false),
+                         RTV(16, false), RTV(24, false), RTV(32, false)};
 #undef RTV
+
+// widest weight of the row instance that d goes to (rt_dispatch)
+int rt_width(int d, bool exact) {
+    if (exact) return d;
+    for (int w : {4, 6, 8, 10, 12, 16, 20, 24})
+        if (d <= w) return w;
+    return 32;
+}
 
 }  // namespace
 
-rt_fn rt_kernel_for(int dmax, bool quirk, bool rsmem) {
+rt_fn rt_kernel_for(int dmax, bool exact, bool quirk, bool rsmem) {
     for (const RtVariant& v : kRt)
-        if (v.dmax == dmax && v.quirk == quirk && v.rsmem == rsmem) return v.k;
+        if (v.dmax == dmax && v.exact == (exact && dmax <= 12) && v.quirk == quirk && v.rsmem == rsmem) return v.k;
     return nullptr;
+}
+
+// Instances of one weight each where a run of layers of equal weight is three layers
+// or longer on average (us, 300 codewords, one weight / two: 802.11n 2/3 Z = 54, one
+// run of eight, 58 / 64; 802.11ay 1/2, 4 runs of 16 layers, 75 / 81; 802.11n 1/2
+// Z = 54, 5 of 12, 81 / 75, and Z = 27, 8 of 12, 114 / 93; 5G NR n1000, 8 of 10, 85 / 75).
+bool rt_exact(const ldpc_code& c) {
+    if (c.max_row_weight > 12) return false;
+    int runs = 1;
+    for (int l = 1; l < c.mrow; ++l) runs += c.row_weights[l] != c.row_weights[l - 1];
+    return 3 * runs <= c.mrow;
 }
 
 // posterior stride: n rounded so that stride mod 32 = ceil(32/G)
@@ -72,7 +93,8 @@ int rt_default_G(int z, int n) {
 
 int rt_dmax(int d) { return d <= 8 ? 8 : d <= 12 ? 12 : d <= 16 ? 16 : d <= 24 ? 24 : d <= 32 ? 32 : 0; }
 
-int make_rt_code(const ldpc_code& c, int max_iter, uint32_t maxv2, const int* beta8, int beta8_all, int G, RtCode* out) {
+int make_rt_code(const ldpc_code& c, int max_iter, uint32_t maxv2, const int* beta8, int beta8_all, int G, bool exact,
+                 RtCode* out) {
     const int E = (int)c.row_cols.size();
     if (c.mrow > RT_MAX_L || E > RT_MAX_E)
         return fail(LDPC_ERR_UNSUPPORTED, "int8 decoder: %d layers / %d circulants exceed %d / %d", c.mrow, E, RT_MAX_L,
@@ -105,7 +127,7 @@ int make_rt_code(const ldpc_code& c, int max_iter, uint32_t maxv2, const int* be
         e0 += c.row_weights[l];
     }
     for (int l = c.mrow - 1; l >= 0; --l)
-        r.run[l] = l + 1 < c.mrow && r.rw[l + 1] == r.rw[l] ? r.run[l + 1] : (int16_t)(l + 1);
+        r.run[l] = l + 1 < c.mrow && rt_width(r.rw[l + 1], exact) == rt_width(r.rw[l], exact) ? r.run[l + 1] : (int16_t)(l + 1);
     for (int e = 0; e < E; ++e)
         r.edge[e] = {4u * (uint32_t)(c.row_cols[e] * c.z), 4u * (uint32_t)(c.row_shifts[e] - c.z)};
     return LDPC_OK;
@@ -141,7 +163,7 @@ int setup_oms_rt(ldpc_ctx* x) {
         return fail(LDPC_ERR_UNSUPPORTED, "int8 decoder: N=%d needs %zu B of shared memory", n, smem);
     RtCode host;
     const int* table = x->layer_beta8.empty() ? nullptr : x->layer_beta8.data();
-    int rc = make_rt_code(c, (int)x->cfg.max_iter, x->maxv2, table, (int)(int8_t)x->cfg.beta, G, &host);
+    int rc = make_rt_code(c, (int)x->cfg.max_iter, x->maxv2, table, (int)(int8_t)x->cfg.beta, G, rt_exact(c), &host);
     if (rc) return rc;
     if (x->tab_rows) {
         std::vector<uint16_t> h(x->tab_beta8.size());
@@ -151,7 +173,7 @@ int setup_oms_rt(ldpc_ctx* x) {
         host.beta_tab = x->d_beta_tab;
         host.tab_rows = x->tab_rows;
     }
-    rt_fn k = rt_kernel_for(dmax, quirk, rsmem);
+    rt_fn k = rt_kernel_for(dmax, rt_exact(c), quirk, rsmem);
     CUDA_TRY(allow_dynamic_smem((const void*)k, kRtMaxSmem));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, threads, smem));

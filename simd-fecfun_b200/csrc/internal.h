@@ -194,8 +194,11 @@ int launch_oms(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s);
 int setup_oms_rt(ldpc_ctx* x);
 int launch_oms_rt(ldpc_ctx* x, const DecodeArgs& a, cudaStream_t s);
 // Fill `out` for one code: int8 offset beta8[l] per layer (nullptr: beta8_all on every
-// layer), Max8 as half2 bits, G quads of codewords per CTA.
-int make_rt_code(const ldpc_code& c, int max_iter, uint32_t maxv2, const int* beta8, int beta8_all, int G, RtCode* out);
+// layer), Max8 as half2 bits, G quads of codewords per CTA, exact as the kernel that decodes it.
+int make_rt_code(const ldpc_code& c, int max_iter, uint32_t maxv2, const int* beta8, int beta8_all, int G, bool exact,
+                 RtCode* out);
+// 1: the kernels with a row instance for every weight, 0: for several neighbouring ones
+bool rt_exact(const ldpc_code& c);
 // Largest row weight the run-time kernels unroll for (0: unsupported).
 int rt_dmax(int max_row_weight);
 // quads of codewords per CTA of the run-time-table kernel for a code of lift Z
@@ -203,7 +206,7 @@ int rt_dmax(int max_row_weight);
 int rt_default_G(int z, int n);
 constexpr int kRtMaxThreads = 512;          // __launch_bounds__ of oms_rt_kernel
 constexpr int kRtMaxSmem = 206 * 1024;      // dynamic shared memory the run-time kernels may use
-rt_fn rt_kernel_for(int dmax, bool quirk, bool rsmem);
+rt_fn rt_kernel_for(int dmax, bool exact, bool quirk, bool rsmem);   // exact: of widths up to 12
 constexpr int kRtMaxG = 8;                  // quads per CTA: 32 codeword slots, one per lane
 int rt_stride(int n, int G);
 // dynamic shared memory of one CTA: tables, G quads of posteriors and staging, messages if rsmem

@@ -10,7 +10,7 @@
 //     every address, table word, load, store and the syndrome's XOR is shared
 //     by four codewords;
 //   - the layer loop over tables in shared memory (row weights and
-//     circulants), rows as straight-line code per weight;
+//     circulants), rows as straight-line code (rt_dispatch);
 //   - the offset beta8 per layer (a single beta is the reference's case; a
 //     table of offsets serves learned offsets);
 //   - the check messages in shared memory (RSMEM) or, for large codes, in a
@@ -25,12 +25,14 @@
 // syndrome and of the slot phase.  Against two codewords per word and a test per
 // edge (73 warp instructions per pair's edge in all, issue 53 %):
 //   802.11n 2/3 Z = 81, 33333 codewords   1.55 -> 1.02 ms
-//   5G NR base graph 1, Z = 384, 6001     11.5 -> 6.5 ms
-//   18 802.11 codes, 50000 each           24.0 -> 20.2 ms
+//   5G NR base graph 1, Z = 384, 6001     11.5 -> 6.4 ms
+//   18 802.11 codes, 50000 each           24.0 -> 15.4 ms
 // of which in the same order: four per word 1.55 -> 1.29, constants in registers
 // (no change at 12 warps), rows and syndrome by runs of one weight, messages of a
 // new codeword masked instead of cleared, counters in registers, 32-bit indices
-// 1.29 -> 1.03 (5G: 9.7 -> 7.5), wide loads from global memory 7.5 -> 6.5.
+// 1.29 -> 1.03 (5G: 9.7 -> 7.5), wide loads from global memory 7.5 -> 6.6 (reads of
+// finished codewords before refills: 6.7), row instances shared by neighbouring
+// weights 6.7 -> 6.4 (802.11 codes: 20.4 -> 15.4).
 #pragma once
 #include <stddef.h>
 
@@ -56,11 +58,21 @@ __device__ __forceinline__ void rt_offsets(const RtCode& C, int l, int it0, int 
     quirk = (b0 ? 0u : 0x0000d800u) | (b1 ? 0u : 0xd8000000u);
 }
 
-// Row weights of a launch's codes go to an unrolled width: each weight up to
-// 12 by itself, then pairs, then fours (f(lo, w): lo <= d <= w).  d is the
-// same for every thread of the CTA, so the branch is uniform; inside, a row
-// is straight-line code.
-template <int DMAX, class F>
+// Rows run as straight-line code, one instance per width: f(lo, w) is called
+// with the instance of weights lo <= d <= w.  d is the same for every thread of
+// the CTA, so the branch is uniform.
+//
+// A row's code is about 700 bytes per edge, so what an SM executes in an
+// iteration may not stay in its instruction caches: a layer that goes to
+// another instance than the one before waits for instructions (802.11ad 13/16,
+// weights 14, 15 and 16, three layers: 6300 cycles with an instance for every
+// two weights, 3700 with one for all three).  Two sets of kernels, so that the
+// unused instances of one do not spread the code of the other apart:
+//   EXACT   an instance for each weight up to 12: codes whose layers come in runs
+//           of a weight (rt_exact)
+//   !EXACT  an instance for two neighbouring weights up to 12, four up to 24, eight
+//           above, with tests for the edges that not all of them have: other codes
+template <int DMAX, bool EXACT, class F>
 __device__ __forceinline__ void rt_dispatch(int d, F&& f) {
 #define RT_WIDTH(LO, W)                                                                   \
     if constexpr (DMAX >= W) {                                                            \
@@ -69,9 +81,14 @@ __device__ __forceinline__ void rt_dispatch(int d, F&& f) {
             return;                                                                       \
         }                                                                                 \
     }
-    RT_WIDTH(2, 2) RT_WIDTH(3, 3) RT_WIDTH(4, 4) RT_WIDTH(5, 5) RT_WIDTH(6, 6) RT_WIDTH(7, 7) RT_WIDTH(8, 8)
-    RT_WIDTH(9, 9) RT_WIDTH(10, 10) RT_WIDTH(11, 11) RT_WIDTH(12, 12) RT_WIDTH(13, 14) RT_WIDTH(15, 16)
-    RT_WIDTH(17, 18) RT_WIDTH(19, 20) RT_WIDTH(21, 22) RT_WIDTH(23, 24) RT_WIDTH(25, 28) RT_WIDTH(29, 32)
+    if constexpr (EXACT) {
+        static_assert(DMAX <= 12);
+        RT_WIDTH(2, 2) RT_WIDTH(3, 3) RT_WIDTH(4, 4) RT_WIDTH(5, 5) RT_WIDTH(6, 6) RT_WIDTH(7, 7) RT_WIDTH(8, 8)
+        RT_WIDTH(9, 9) RT_WIDTH(10, 10) RT_WIDTH(11, 11) RT_WIDTH(12, 12)
+    } else {
+        RT_WIDTH(2, 4) RT_WIDTH(5, 6) RT_WIDTH(7, 8) RT_WIDTH(9, 10) RT_WIDTH(11, 12) RT_WIDTH(13, 16)
+        RT_WIDTH(17, 20) RT_WIDTH(21, 24) RT_WIDTH(25, 32)
+    }
 #undef RT_WIDTH
 }
 
@@ -175,19 +192,20 @@ __device__ __forceinline__ void rt_row(const SpEdge* ed, int d, char* Pg, uint32
 // Syndrome of this thread's check rows with early exit (as oms_syndrome), four
 // codewords at once: bit 7 of a posterior's byte is set where it is not
 // negative, so a check fails where the XOR of its words' bits 7 differs from
-// its weight's parity.  all: bits 7 of the bytes in use.  Two rows of a run of
-// equal weights at a time, so that their loads are in flight together.
-template <int DMAX>
+// its weight's parity.  all: bits 7 of the bytes in use.  EXACT: two rows of a
+// run at a time, so that their loads are in flight together; with short runs the
+// code for a row that is left over costs more than that gains (5G NR n1000, 10
+// rows: 6300 against 4900 cycles).
+template <int DMAX, bool EXACT>
 __device__ __forceinline__ void rt_syndrome(const RtCode& C, char* Pg, uint32_t tb, uint32_t zb, uint32_t all, uint32_t* synd) {
     uint32_t seen = 0;
     for (int l = 0; l < C.L;) {
-        const int d = C.rw[l], end = C.run[l];
+        const int first = C.rw[l], end = C.run[l];
         const SpEdge* ed = C.edge + C.ebase[l];
-        const uint32_t odd = (d & 1) ? 0x80808080u : 0u;
-        rt_dispatch<DMAX>(d, [&](auto lo_, auto w_) {
-            constexpr int LO = decltype(lo_)::value, W = decltype(w_)::value;
-            auto row = [&](const SpEdge* t) {
-                uint32_t x = odd;
+        rt_dispatch<DMAX, EXACT>(first, [&](auto lo_, auto w_) {
+            constexpr int LO = decltype(lo_)::value, W = decltype(w_)::value, STEP = EXACT ? 2 : 1;
+            auto row = [&](const SpEdge* t, int d) {
+                uint32_t x = (d & 1) ? 0x80808080u : 0u;
 #pragma unroll
                 for (int j = 0; j < W; ++j) {
                     const uint32_t v = *rt_at(t[j < LO ? j : min(j, d - 1)], Pg, tb, zb);
@@ -196,7 +214,8 @@ __device__ __forceinline__ void rt_syndrome(const RtCode& C, char* Pg, uint32_t 
                 return x;
             };
             do {
-                uint32_t x = l + 1 < end ? row(ed) | row(ed + d) : row(ed);
+                const int d = LO == W ? W : C.rw[l];
+                uint32_t x = STEP == 2 && l + 1 < end ? row(ed, W) | row(ed + W, W) : row(EXACT ? ed : C.edge + C.ebase[l], d);
                 x &= all;
                 if (x & ~seen) {
                     atomicOr(synd, x);
@@ -206,8 +225,8 @@ __device__ __forceinline__ void rt_syndrome(const RtCode& C, char* Pg, uint32_t 
                     l = C.L;
                     return;
                 }
-                ed += 2 * d;
-                l += 2;
+                ed += STEP * W;
+                l += STEP;
             } while (l < end);
             l = end;
         });
@@ -417,7 +436,7 @@ __device__ __forceinline__ void rt_slots_coop(const RtCode& C, const RtJob& job,
     }
 }
 
-template <int DMAX, bool QUIRK, bool RSMEM>
+template <int DMAX, bool EXACT, bool QUIRK, bool RSMEM>
 __global__ void __launch_bounds__(512) oms_rt_kernel(const __grid_constant__ RtLaunch lp) {
     extern __shared__ __align__(16) unsigned char rt_smem[];
     __shared__ long long s_cur[32];
@@ -545,12 +564,12 @@ __global__ void __launch_bounds__(512) oms_rt_kernel(const __grid_constant__ RtL
             for (int k = 0; k < 4; ++k)
                 its[k] = active && k < (1 << sh) ? max(s_it[par][(g << sh) + k], 0) : 0;
             for (int l = 0; l < C.L;) {
-                // a run of layers of one weight
-                const int d = C.rw[l], end = C.run[l];
+                // a run of layers of one instance
+                const int first = C.rw[l], end = C.run[l];
                 auto rows = [&](auto lo_, auto w_, auto nh_) {
                     do {
                         if (active) {
-                            const int eb = C.ebase[l];
+                            const int eb = C.ebase[l], d = C.rw[l];
                             uint32_t beta2[2], quirk[2];
                             rt_offsets(C, l, its[0], its[1], beta2[0], quirk[0]);
                             rt_offsets(C, l, its[2], its[3], beta2[1], quirk[1]);
@@ -561,16 +580,16 @@ __global__ void __launch_bounds__(512) oms_rt_kernel(const __grid_constant__ RtL
                     } while (++l < end);
                 };
                 if (lp.half)
-                    rt_dispatch<DMAX>(d, [&](auto lo_, auto w_) { rows(lo_, w_, std::integral_constant<int, 1>{}); });
+                    rt_dispatch<DMAX, EXACT>(first, [&](auto lo_, auto w_) { rows(lo_, w_, std::integral_constant<int, 1>{}); });
                 else
-                    rt_dispatch<DMAX>(d, [&](auto lo_, auto w_) { rows(lo_, w_, std::integral_constant<int, 2>{}); });
+                    rt_dispatch<DMAX, EXACT>(first, [&](auto lo_, auto w_) { rows(lo_, w_, std::integral_constant<int, 2>{}); });
             }
             if (tid < 16) {
                 s_synd[par ^ 1][tid] = 0;
                 s_zero_mask[par ^ 1][tid] = 0;
             }
             if (tid == 0) s_busy[par ^ 1] = 0;
-            if (active) rt_syndrome<DMAX>(C, Pg, tb, zb, in_use, &s_synd[par][g]);
+            if (active) rt_syndrome<DMAX, EXACT>(C, Pg, tb, zb, in_use, &s_synd[par][g]);
             cp_async_wait_all();   // this thread's prefetches (issued in an earlier slot phase)
             __syncthreads();       // syndrome bits final, every prefetched byte visible
 

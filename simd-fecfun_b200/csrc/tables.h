@@ -111,7 +111,7 @@ struct alignas(16) RtCode {
     int tab_rows;                    //   (0-based) uses row min(i, tab_rows - 1), in place of beta2 / quirk2
     int16_t rw[RT_MAX_L];
     int16_t ebase[RT_MAX_L];         // first edge of layer l
-    int16_t run[RT_MAX_L];           // first layer after l of another weight (or L)
+    int16_t run[RT_MAX_L];           // first layer after l of another row instance (or L)
     SpEdge edge[RT_MAX_E];           // in bytes of a posterior word; a CTA copies E of them
 };
 
