@@ -656,26 +656,38 @@ __global__ void __launch_bounds__(256) encode_kernel(const __grid_constant__ Gen
             }
             __syncwarp();
         }
-        uint8_t* const dst = cw_out + i0 * tb.n;
-        for (int j = lane, c = 0, q = lane; j < m * nv; j += 32, q += 32) {
-            while (q >= nv) {
-                q -= nv;
-                ++c;
+        uint8_t* dst = cw_out + i0 * tb.n;
+        if constexpr (V == 1) {
+            // unaligned output, a byte per lane: one word each, read without the steps that a store
+            // of several bits needs (5G NR base graph 1, 9000 codewords: 589 -> 346 us)
+            for (int c = 0; c < m; ++c, dst += tb.n) {
+                const uint32_t* const w = mine + c * sh.stride;
+#pragma unroll 4
+                for (int i = lane; i < tb.n; i += 32) {
+                    const int col = (int)__umulhi(2u * (uint32_t)i, sh.inv_z), p = i - col * z;
+                    dst[i] = (uint8_t)((w[col * (zw + 1) + (p >> 5)] >> (p & 31)) & 1u);
+                }
             }
-            const int idx = V * q, col = (int)__umulhi(2u * (uint32_t)idx, sh.inv_z), p = idx - col * z;
-            const uint32_t* w = mine + c * sh.stride + col * (zw + 1);
-            uint32_t v = stream_bits32(w, p);
-            for (int have = z - p; have < V; have += z) {
-                w += zw + 1;
-                v |= w[0] << have;
-            }
-            uint32_t o[(V + 3) / 4];
+        } else {
+            for (int j = lane, c = 0, q = lane; j < m * nv; j += 32, q += 32) {
+                while (q >= nv) {
+                    q -= nv;
+                    ++c;
+                }
+                const int idx = V * q, col = (int)__umulhi(2u * (uint32_t)idx, sh.inv_z), p = idx - col * z;
+                const uint32_t* w = mine + c * sh.stride + col * (zw + 1);
+                uint32_t v = stream_bits32(w, p);
+                for (int have = z - p; have < V; have += z) {
+                    w += zw + 1;
+                    v |= w[0] << have;
+                }
+                uint32_t o[(V + 3) / 4];
 #pragma unroll
-            for (int b = 0; b < (V + 3) / 4; ++b) o[b] = (((v >> (4 * b)) & 15u) * 0x00204081u) & 0x01010101u;
-            if (V == 16) *reinterpret_cast<uint4*>(dst + V * j) = make_uint4(o[0], o[V > 4], o[2 * (V > 8)], o[3 * (V > 8)]);
-            else if (V == 8) *reinterpret_cast<uint2*>(dst + V * j) = make_uint2(o[0], o[V > 4]);
-            else if (V == 4) *reinterpret_cast<uint32_t*>(dst + V * j) = o[0];
-            else dst[j] = (uint8_t)(v & 1u);
+                for (int b = 0; b < (V + 3) / 4; ++b) o[b] = (((v >> (4 * b)) & 15u) * 0x00204081u) & 0x01010101u;
+                if (V == 16) *reinterpret_cast<uint4*>(dst + V * j) = make_uint4(o[0], o[V > 4], o[2 * (V > 8)], o[3 * (V > 8)]);
+                else if (V == 8) *reinterpret_cast<uint2*>(dst + V * j) = make_uint2(o[0], o[V > 4]);
+                else *reinterpret_cast<uint32_t*>(dst + V * j) = o[0];
+            }
         }
     }
 }
