@@ -17,7 +17,10 @@ int fail(int code, const char* fmt, ...);
 #define CUDA_TRY(expr)                                                                                    \
     do {                                                                                                  \
         cudaError_t e_ = (expr);                                                                          \
-        if (e_ != cudaSuccess) return ::ldpc::fail(LDPC_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_)); \
+        if (e_ != cudaSuccess) {                                                                          \
+            cudaGetLastError(); /* the next call's launch check does not see it */                        \
+            return ::ldpc::fail(LDPC_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_));                  \
+        }                                                                                                 \
     } while (0)
 
 typedef void (*oms_fn)(const OmsTables, const OmsJob);

@@ -67,3 +67,42 @@ def test_small_host_calls_of_wider_types(capi, kind, outputs):
         assert post is None or np.array_equal(post.view(np.uint8), p.cpu().numpy().view(np.uint8))
         assert hard is None or np.array_equal(hard, h.cpu().numpy())
         assert iters is None or np.array_equal(iters, it.cpu().numpy())
+
+
+@pytest.mark.parametrize("where", ["pinned", "pinned in", "pinned out", "device", "device in", "device out"])
+@pytest.mark.parametrize("n", [1, 40, 60, 187])
+def test_small_host_calls_from_other_memory(capi, n, where):
+    """Page-locked buffers on either side of the size up to which they are moved
+    by memcpy (32 KB: 48 codewords' LLRs), and device memory given as a host buffer, which is
+    an error or decodes as from the host, but is not touched by it."""
+    import torch
+    from ldpc_b200 import codes
+    code = codes.make_code("11ad 1/2")
+    ctx = capi.Context(capi.Code.from_tables(code))
+    llr = torch.empty((1, n, code.n), dtype=torch.int8, device="cuda")
+    ctx.generate(n, 0, [-0.75], n, llr_int=llr)
+    want = (torch.empty_like(llr), torch.empty((n, 11), dtype=torch.int32, device="cuda"),
+            torch.empty(n, dtype=torch.uint8, device="cuda"))
+    ctx.decode_int8(llr, n, post=want[0], hard=want[1], iters=want[2])
+    torch.cuda.synchronize()
+    kind, _, part = where.partition(" ")
+    other = (lambda t: t.pin_memory()) if kind == "pinned" else (lambda t: t.cuda())
+    src = llr.cpu() if part == "out" else other(llr.cpu())
+    outs = [torch.zeros_like(t, device="cpu") if part == "in" else other(torch.zeros_like(t, device="cpu")) for t in want]
+    torch.cuda.synchronize()
+    for some in ((0, 1, 2), (1, 2), (0,), ()):
+        for t in outs:
+            t.zero_()
+        torch.cuda.synchronize()
+        tot = C.c_uint64()
+        ptr = [outs[i].data_ptr() if i in some else None for i in range(3)]
+        rc = capi.lib.ldpc_decode_int8_host(ctx.h, src.data_ptr(), n, *ptr, C.byref(tot))
+        if kind == "device" and rc == capi.LDPC_ERR_CUDA:
+            # the context stays usable
+            got = ctx.decode_host(llr[0].cpu().numpy())
+            assert np.array_equal(got[0], want[0][0].cpu().numpy())
+            continue
+        capi.check(rc)
+        assert tot.value == int(want[2].sum(dtype=torch.int64))
+        for i in some:
+            assert torch.equal(outs[i].cpu(), want[i].cpu())
