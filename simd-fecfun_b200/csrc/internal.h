@@ -73,11 +73,18 @@ inline long long spread_ctas(size_t n, long long slots, int sms) {
 // tanh/atanh chains are latency-bound, so resident warps count for more than
 // message latency, but one CTA more out of five does not pay for the L2 round
 // trips (802.11ad float 26.1e6 against 24.8e6 codewords/s).
-//   Min-sum: unless they give at least 2.5 times.  Light on arithmetic, it takes
-// that many more warps to cover the round trips (Mcw/s, shared against global:
-// float 802.11ad 63.7 / 53.8, 802.11n 2/3 Z = 81 14.1 / 13.7, 802.11ay 1/2
-// 16.9 / 23.9, 5G NR n6400 1.47 / 3.00; double 802.16e Z = 96 4.5 / 6.4,
-// 802.11ad 28.5 / 37.6).
+//   Min-sum and integers: unless they give at least 2.5 times.  Light on arithmetic,
+// they take that many more warps to cover the round trips (ms, shared / global, and the
+// CTAs per SM):
+//   float   802.11ad 1/2 0.66 / 0.77 (5, 5), 802.11n 2/3 Z = 81 2.79 / 2.98 (4, 5),
+//           802.11ay 1/2 2.27 / 1.64 (2, 5), 5G NR n6400 4.95 / 2.46 (1, 4)
+//   double  802.11ad 1/2 1.34 / 1.04 (2, 5), 13/16 0.64 / 0.63 (2, 4), 802.16e Z = 24 1.87 / 0.98 (1, 4)
+//   int16   802.11ad 1/2 0.79 / 0.80 (5, 8), 802.11n 1/2 Z = 27 1.19 / 1.05 (3, 8),
+//           802.11ay 1/2 2.64 / 1.82 (2, 8), 5G NR n6400 5.77 / 2.97 (1, 4)
+//   int32   802.11ad 1/2 0.84 / 0.86 (5, 8), 802.11n 1/2 Z = 27 1.25 / 1.17 (3, 8),
+//           802.11ay 1/2 2.76 / 2.04 (2, 6), 5G NR n6400 6.10 / 3.25 (1, 4)
+// Between 1.6 and 2 times it goes either way by up to 7 % (float 802.11n 1/2 Z = 27
+// 1.03 / 0.96, G.hn 0.41 / 0.42, both 3, 5).
 inline bool messages_in_smem(bool prod, int per_s, int per_g) { return 2 * per_g < (prod ? 3 : 5) * per_s; }
 
 // CTAs that a context's or plan's launches may have: all that the device holds,

@@ -60,14 +60,12 @@ __device__ __forceinline__ uint32_t hmin2(uint32_t a, uint32_t b) { uint32_t d; 
 __device__ __forceinline__ uint32_t hmax2(uint32_t a, uint32_t b) { uint32_t d; asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 __device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c) { uint32_t d; asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
 // 0xffff in each lane where a == b, else 0
-__device__ __forceinline__ uint32_t heq2_mask(uint32_t a, uint32_t b) { uint32_t d; asm("set.eq.u32.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 // 1.0 in each lane where a == b, else 0.0
 __device__ __forceinline__ uint32_t heq2(uint32_t a, uint32_t b) { uint32_t d; asm("set.eq.f16x2.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 __device__ __forceinline__ uint32_t habs2(uint32_t a) { return a & 0x7fff7fffu; }
 // min / max of the magnitudes, with the XOR of the two sign bits as sign:
 // one instruction for |.|, the running minimum and the running sign product
 __device__ __forceinline__ uint32_t hmin2_xs(uint32_t a, uint32_t b) { uint32_t d; asm("min.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
-__device__ __forceinline__ uint32_t hmax2_xs(uint32_t a, uint32_t b) { uint32_t d; asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 
 // max(a * b + c, 0)
 __device__ __forceinline__ uint32_t hfma2_relu(uint32_t a, uint32_t b, uint32_t c) { uint32_t d; asm("fma.rn.relu.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }

@@ -338,7 +338,7 @@ def learned_run(train_steps: int = 30, batch: int = 65536, eval_n: int = 200_000
         "config": {"workload": "802.16e 1/2 Z=96 (N=2304), batches of %d codewords, Eb/N0 uniform in [1.0, 2.5] dB "
                                "(16 points per batch), 120 offsets from 0.5, Adam lr 0.01, BCE over all iterations "
                                "(%s weights)" % (batch, weights),
-                   "step": "generation + encoding + forward with checkpoints + adjoint + Adam"},
+                   "step": "generation + encoding + loss and offset gradient + Adam"},
         "forward_adjoint_ms": fb_ms,
         "forward_adjoint_cw_s": batch / (fb_ms * 1e-3),
         "loss_first_last": [hist[0], hist[-1]],
