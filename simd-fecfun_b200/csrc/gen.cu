@@ -159,8 +159,8 @@ int launch_gen(ldpc_ctx* x, uint64_t seed, uint64_t cw_offset, const float* snr_
     job.uncoded = uncoded;
     GenTile tile;
     const size_t smem = gen_tile_shape(x->gent, &tile);
-    // int8 output alone, whole 4-element blocks, a clamp bound the rounding trick covers
-    tile.fast = (job.llr_i8 && !job.llr_f32 && !job.llr_i16 && !job.llr_i32 && !job.llr_f64 && (x->gent.n & 3) == 0 &&
+    // int8 output alone, aligned and whole 4-element blocks, a clamp bound the rounding trick covers
+    tile.fast = (job.llr_i8 && ((uintptr_t)job.llr_i8 & 3) == 0 && !job.llr_f32 && !job.llr_i16 && !job.llr_i32 && !job.llr_f64 && (x->gent.n & 3) == 0 &&
                  std::fabs(job.max_abs) < 32767.0f && n_snr <= (size_t)GEN_FAST_SNR) ? 1 : 0;
     // the 16-bit clamp after rounding needs |rx * sf| < 2^15 before the clamp: |noise| <= 9.5 (the
     // generator's largest Box-Muller radius), so |rx| <= 1 + 9.5 sigma

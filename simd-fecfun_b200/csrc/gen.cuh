@@ -474,10 +474,11 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
             // (c, b) of item f advanced by GEN_THREADS items per step, without a division per item
             int c = tid / nb, b = tid - (tid / nb) * nb;
             const int step_c = GEN_THREADS / nb, step_b = GEN_THREADS - step_c * nb;
-            // 16-byte stores of wider integers and doubles: whole blocks, aligned output
+            // stores of several elements: whole blocks of aligned outputs
             const unsigned long long at = reinterpret_cast<unsigned long long>(job.llr_i16) | reinterpret_cast<unsigned long long>(job.llr_i32) |
-                                          reinterpret_cast<unsigned long long>(job.llr_f64);
+                                          reinterpret_cast<unsigned long long>(job.llr_f64) | reinterpret_cast<unsigned long long>(job.llr_f32);
             const bool wide = ((tb.n & 3) | (int)(at & 15)) == 0;
+            const bool wide8 = ((tb.n & 3) | (int)(reinterpret_cast<unsigned long long>(job.llr_i8) & 3)) == 0;
             for (int f = tid; f < tc * nb; f += GEN_THREADS, c += step_c, b += step_b) {
                 if (b >= nb) {
                     b -= nb;
@@ -522,7 +523,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
 #pragma unroll
                         for (int q = 0; q < 4; ++q) packed |= (uint32_t)(uint8_t)llr_to_i8(l[q]) << (8 * q);
                         int8_t* dst = job.llr_i8 + row * tb.n + idx0;
-                        if ((tb.n & 3) == 0) {
+                        if (wide8) {
                             *reinterpret_cast<uint32_t*>(dst) = packed;
                         } else {
                             for (int q = 0; q < 4 && idx0 + q < tb.n; ++q) dst[q] = (int8_t)(packed >> (8 * q));
@@ -560,7 +561,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 4) gen_kernel(const __grid_consta
                     }
                     if (job.llr_f32) {
                         float* dst = job.llr_f32 + row * tb.n + idx0;
-                        if ((tb.n & 3) == 0) {
+                        if (wide) {
                             *reinterpret_cast<float4*>(dst) = make_float4(l[0], l[1], l[2], l[3]);
                         } else {
                             for (int q = 0; q < 4 && idx0 + q < tb.n; ++q) dst[q] = l[q];

@@ -283,3 +283,27 @@ def test_encode_narrow_columns(capi, oracle, z, name, offset):
         got = out.cpu().numpy()
         assert np.array_equal(got[offset:offset + n * code.n].reshape(n, code.n), oracle.encode(code, info))
         assert (got[:offset] == 7).all() and (got[offset + n * code.n:] == 7).all()
+
+
+@pytest.mark.parametrize("outputs", ["i8", "f32", "both"])
+@pytest.mark.parametrize("name,n", [("11ad 1/2", 3), ("11ad 1/2", 700), ("ITU G.hn 1/2 z14", 40), ("5GNR_n3136_k576", 40)])
+def test_unaligned_outputs(capi, name, n, outputs):
+    """int8 LLRs at a base that is not a multiple of 4 bytes and float ones at one
+    that is not of 16 are those of aligned bases; bytes around them stay."""
+    import torch
+    from ldpc_b200 import codes
+    code = capi.Code.from_tables(codes.code_by_name(name))
+    ctx = capi.Context(code, max_iter=2, llr_scale=2.0, max_abs_llr=24.0)
+    snrs, N = [-1.0, 0.0], code.info.n
+    kinds = {"i8": torch.int8, "f32": torch.float32}
+    used = list(kinds) if outputs == "both" else [outputs]
+    want, unc = {k: torch.empty((2, n, N), dtype=kinds[k], device="cuda") for k in used}, torch.zeros((4, 2), dtype=torch.int64, device="cuda")
+    ctx.generate(9, 5, snrs, n, uncoded=unc[0], **{"llr_" + k: want[k] for k in used})
+    for offset in (1, 2, 3):
+        buf = {k: torch.full((2 * n * N + 8,), 77, dtype=kinds[k], device="cuda") for k in used}
+        ctx.generate(9, 5, snrs, n, uncoded=unc[offset], **{"llr_" + k: buf[k].data_ptr() + offset * buf[k].element_size() for k in used})
+        torch.cuda.synchronize()
+        for k in used:
+            assert torch.equal(buf[k][offset:offset + want[k].numel()].view(want[k].shape), want[k])
+            assert (buf[k][:offset] == 77).all() and (buf[k][offset + want[k].numel():] == 77).all()
+        assert torch.equal(unc[offset], unc[0])
