@@ -514,23 +514,14 @@ int decode_host_small(ldpc_ctx* x, const T* llr, size_t n, T* post, uint32_t* ha
         bool move;
     };
     Out out[3] = {{post, in_bytes, 0, true}, {hard, n * (size_t)x->hard_words * 4, 0, true}, {iters, n, 0, true}};
-    // on the device: LLRs, outputs with a copy of their own, outputs that share one (iterations always do)
-    size_t end = 0;
-    auto take = [&](size_t b) {
-        const size_t at = end;
-        end += (b + 255) & ~(size_t)255;
-        return at;
-    };
-    take(in_bytes);
-    for (Out& o : out)
-        if (o.dst) o.move = by_memcpy(o.dst, o.bytes);
-    for (int i = 0; i < 2; ++i)
-        if (out[i].dst && !out[i].move) out[i].at = take(out[i].bytes);
-    const size_t shared = end;
-    for (int i = 0; i < 2; ++i)
-        if (out[i].dst && out[i].move) out[i].at = take(out[i].bytes);
-    out[2].at = end;
-    end += n;
+    // on the device as in the pinned buffer: LLRs, then the outputs that are asked for, then iterations
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    size_t end = up(in_bytes);
+    for (Out& o : out) {
+        o.at = end;
+        end += o.dst ? up(o.bytes) : 0;
+    }
+    end = out[2].at + n;
     void* d = nullptr;
     if (int rc = pipe_buffer(x, 0, 0, ldpc_ctx::kSmallHost, &d)) return rc;
     uint8_t *h = x->h_small, *dev = (uint8_t*)d;
@@ -546,8 +537,15 @@ int decode_host_small(ldpc_ctx* x, const T* llr, size_t n, T* post, uint32_t* ha
         a.hard = hard ? (uint32_t*)(dev + out[1].at) : nullptr;
         a.iters = dev + out[2].at;
         if (int rc = ldpc::launch_decode(x, a, s)) return rc;
-        for (const Out& o : out)
-            if (o.dst && !o.move) CUDA_TRY(cudaMemcpyAsync(o.dst, dev + o.at, o.bytes, cudaMemcpyDeviceToHost, s));
+        // the outputs' kind of memory while the device works
+        size_t shared = out[2].at;   // start of the common copy: the first output that is moved
+        for (int i = 2; i >= 0; --i) {
+            Out& o = out[i];
+            if (!o.dst) continue;
+            o.move = by_memcpy(o.dst, o.bytes);
+            if (o.move) shared = o.at;
+            else CUDA_TRY(cudaMemcpyAsync(o.dst, dev + o.at, o.bytes, cudaMemcpyDeviceToHost, s));
+        }
         CUDA_TRY(cudaMemcpyAsync(h + shared, dev + shared, end - shared, cudaMemcpyDeviceToHost, s));
         return LDPC_OK;
     };
